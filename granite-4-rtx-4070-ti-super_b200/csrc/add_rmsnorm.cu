@@ -310,6 +310,16 @@ __global__ void __launch_bounds__(256) add_rmsnorm_fast_kernel(const NormParams 
   }
 }
 
+// bf16(h * r * w) of eight packed values, products rounded one after the other.
+__device__ __forceinline__ uint32_t norm_pair(uint32_t h, F32x2 r, F32x2 w) {
+  float a, b;
+  f32x2_split(mul2(mul2(bf16x2_f32(h), r), w), a, b);
+  return pack_bf16x2(a, b);
+}
+__device__ __forceinline__ uint4 norm8(uint4 h, F32x2 r, const F32x2 (&w)[4]) {
+  return make_uint4(norm_pair(h.x, r, w[0]), norm_pair(h.y, r, w[1]), norm_pair(h.z, r, w[2]), norm_pair(h.w, r, w[3]));
+}
+
 // Second sweep with r known per row: a plain streaming pass. A CTA takes kRowsPerCta
 // consecutive rows; a thread takes the chunks t, t + T, ... of each, so every
 // thread has kRowsPerCta * ceil(cols8 / T) independent 128-bit loads to issue
@@ -358,16 +368,12 @@ __global__ void __launch_bounds__(kEncodeThreads) norm_encode_kernel(const NormP
     for (int k = 0; k < kEncodeMaxIter; ++k) {
       const int c = c0 + k * kEncodeThreads + t;
       if (!FULL && c >= p.cols8) continue;
-      float wf[8];
-      unpack8(wv[k], wf);  // once per column chunk, shared by the rows
+      const F32x2 w2[4] = {bf16x2_f32(wv[k].x), bf16x2_f32(wv[k].y), bf16x2_f32(wv[k].z), bf16x2_f32(wv[k].w)};
 #pragma unroll
       for (int j = 0; j < kRowsPerCta; ++j) {
         if (!FULL && row0 + j >= p.rows) continue;
-        float hf[8], n[8];
-        unpack8(hv[j][k], hf);
-#pragma unroll
-        for (int e = 0; e < 8; ++e) n[e] = __fmul_rn(__fmul_rn(hf[e], rr[j]), wf[e]);
-        st_stream(out + static_cast<size_t>(row0 + j) * p.cols8 + c, fp8x8_quant(pack8(n), fs));
+        const F32x2 r2 = f32x2(rr[j], rr[j]);
+        st_stream(out + static_cast<size_t>(row0 + j) * p.cols8 + c, fp8x8_quant(norm8(hv[j][k], r2, w2), fs));
       }
     }
   }
