@@ -63,9 +63,17 @@ struct NormParams {
   double inv_cols;  // 1 / cols when cols is a power of two (the scaling is then exact), else 0
 };
 
-// kCluster: the whole grid is one cluster of at most 16 CTAs with one row each; stats and encode in
-// one launch (g4_cluster.cuh).
-enum { kStats = 0, kEncode = 1, kCluster = 2 };
+enum { kStats = 0, kEncode = 1 };
+
+// bf16(h * r * w) of eight packed values, products rounded one after the other.
+__device__ __forceinline__ uint32_t norm_pair(uint32_t h, F32x2 r, F32x2 w) {
+  float a, b;
+  f32x2_split(mul2(mul2(bf16x2_f32(h), r), w), a, b);
+  return pack_bf16x2(a, b);
+}
+__device__ __forceinline__ uint4 norm8(uint4 h, F32x2 r, const F32x2 (&w)[4]) {
+  return make_uint4(norm_pair(h.x, r, w[0]), norm_pair(h.y, r, w[1]), norm_pair(h.z, r, w[2]), norm_pair(h.w, r, w[3]));
+}
 
 // Load one 8-element chunk as floats.
 template <bool F32>
@@ -87,14 +95,9 @@ template <bool Y_F32, bool RES_F32, int V, int PHASE>
 __global__ void __launch_bounds__(max_threads_for(V))
     add_rmsnorm_kernel(const NormParams p) {
   pdl_begin();
-  if (PHASE == kCluster) cluster_announce();
   const int T = blockDim.x;
   const int t = threadIdx.x;
-  // A cluster is a power of two wide: its spare CTAs redo the last row without storing anything,
-  // so that they reach the cluster barrier with a harmless contribution.
-  const bool live = PHASE != kCluster || static_cast<int>(blockIdx.x) < p.rows;
-  const int row = PHASE == kCluster ? (live ? static_cast<int>(blockIdx.x) : p.rows - 1)
-                                    : (p.reverse ? p.rows - 1 - static_cast<int>(blockIdx.x) : blockIdx.x);
+  const int row = p.reverse ? p.rows - 1 - static_cast<int>(blockIdx.x) : blockIdx.x;
   const size_t row_chunk0 = static_cast<size_t>(row) * p.cols8;
 
   float h[V][8];
@@ -132,7 +135,7 @@ __global__ void __launch_bounds__(max_threads_for(V))
   for (int j = 0; j < V; ++j) {
     const uint4 hb = pack8(h[j]);
     unpack8(hb, h[j]);
-    if (PHASE != kEncode && live && p.h_out != nullptr) {
+    if (PHASE != kEncode && p.h_out != nullptr) {
       const int c = t + j * T;
       // default cache policy: the second sweep re-reads it
       if (c < p.cols8) reinterpret_cast<uint4*>(p.h_out)[row_chunk0 + c] = hb;
@@ -163,13 +166,12 @@ __global__ void __launch_bounds__(max_threads_for(V))
   const float ms = static_cast<float>(p.inv_cols != 0.0 ? total * p.inv_cols
                                                          : total / static_cast<double>(p.cols));
   const float r = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(ms, p.eps)));
-  if (PHASE != kEncode && live && p.rstd != nullptr && t == 0) p.rstd[row] = r;
+  if (PHASE != kEncode && p.rstd != nullptr && t == 0) p.rstd[row] = r;
 
   // ---- normalise -----------------------------------------------------------------
   Fp8Scale fs{};
   if (PHASE == kEncode) fs = fp8_scale_from_amax(__ldcg(p.scale_amax + 1));
   uint32_t amax = 0u;
-  uint4 kept[PHASE == kCluster ? V : 1];  // kCluster: n stays in registers across the barrier
 #pragma unroll
   for (int j = 0; j < V; ++j) {
     const int c = t + j * T;
@@ -179,12 +181,7 @@ __global__ void __launch_bounds__(max_threads_for(V))
 #pragma unroll
       for (int e = 0; e < 8; ++e) n[e] = __fmul_rn(__fmul_rn(h[j][e], r), wv[e]);
       const uint4 nb = pack8(n);
-      if (PHASE == kCluster) {
-        if (live && p.n_bf16 != nullptr)
-          st_stream(reinterpret_cast<uint4*>(p.n_bf16) + row_chunk0 + c, nb);
-        kept[PHASE == kCluster ? j : 0] = nb;
-        amax = amax_acc(amax, nb);
-      } else if (PHASE == kStats) {
+      if (PHASE == kStats) {
         if (p.n_bf16 != nullptr) {
           uint4* dst = reinterpret_cast<uint4*>(p.n_bf16) + row_chunk0 + c;
           if (p.n_fp8 != nullptr) *dst = nb; else st_stream(dst, nb);
@@ -206,20 +203,103 @@ __global__ void __launch_bounds__(max_threads_for(V))
     }
   }
   if (PHASE == kEncode && blockIdx.x == 0 && t == 0) p.scale_amax[0] = fs.scale;
-  if (PHASE == kCluster) {
-    __shared__ uint32_t s_slots[kMaxClusterCtas];
-    const float tensor_amax = __uint_as_float(cluster_amax_bits(amax, s_amax, s_slots));
-    fs = fp8_scale_from_amax(tensor_amax);
-    if (live) {
+}
+
+// At most 16 rows with FP8 output (a decode or verify step): one CTA per row, the rows one thread-block
+// cluster (g4_cluster.cuh; a single row needs none), stats and encode in one launch with the row in
+// registers. What such a launch costs is its own chain of latencies - the launch itself is under a
+// microsecond in a programmatic chain - so: the weights are asked into L2 while the kernel ahead still
+// runs and loaded together with y and res; 256 threads of two chunks each (a 4096-wide row) keep the
+// double-precision sum two chains of eight long and the partial sums few; every later exchange is one
+// shuffle level or one redux. One row of 4096, in a chain of such
+// launches: 2.9 us for the row kernel it replaces, 2.0 now.
+constexpr int kSmallChunks = 2;
+template <bool Y_F32, bool RES_F32, bool CLUSTER>
+__global__ void __launch_bounds__(512) norm_small_kernel(const NormParams p) {
+  const int T = blockDim.x, t = threadIdx.x, lane = t & 31, warp = t >> 5, nwarps = T >> 5;
+  const uint4* w = reinterpret_cast<const uint4*>(p.w);
 #pragma unroll
-      for (int j = 0; j < V; ++j) {
-        const int c = t + j * T;
-        if (c < p.cols8)
-          st_stream(reinterpret_cast<uint2*>(p.n_fp8) + row_chunk0 + c, fp8x8_quant(kept[PHASE == kCluster ? j : 0], fs));
+  for (int j = 0; j < kSmallChunks; ++j)
+    if (t + j * T < p.cols8 && (t & 7) == 0) prefetch_l2(w + t + j * T);
+  pdl_begin();
+  if (CLUSTER) cluster_announce();
+  // A cluster is a power of two wide: its spare CTAs redo the last row without storing anything,
+  // so that they reach the cluster barrier with a harmless contribution.
+  const bool live = !CLUSTER || static_cast<int>(blockIdx.x) < p.rows;
+  const size_t row_chunk0 = static_cast<size_t>(live ? static_cast<int>(blockIdx.x) : p.rows - 1) * p.cols8;
+  float h[kSmallChunks][8], rv[kSmallChunks][8];
+  uint4 wv[kSmallChunks];
+#pragma unroll
+  for (int j = 0; j < kSmallChunks; ++j) {
+    const int c = t + j * T;
+    wv[j] = make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) h[j][e] = rv[j][e] = 0.0f;
+    if (c < p.cols8) {
+      load_chunk<Y_F32>(p.y, row_chunk0 + c, h[j]);
+      if (p.res != nullptr) load_chunk<RES_F32>(p.res, row_chunk0 + c, rv[j]);
+      wv[j] = __ldg(w + c);
+    }
+  }
+  uint4 hb[kSmallChunks];
+  double acc[kSmallChunks];
+#pragma unroll
+  for (int j = 0; j < kSmallChunks; ++j) {
+    if (p.res != nullptr) {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) h[j][e] = __fadd_rn(rv[j][e], __fmul_rn(p.rm, h[j][e]));
+    }
+    hb[j] = pack8(h[j]);
+    unpack8(hb[j], h[j]);
+    acc[j] = 0.0;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const double d = static_cast<double>(h[j][e]);
+      acc[j] = fma(d, d, acc[j]);
+    }
+  }
+  __shared__ double s_part[16];
+  __shared__ uint32_t s_amax[16];
+  const double sum = warp_sum(acc[0] + acc[1]);
+  if (lane == 0) s_part[warp] = sum;
+  __syncthreads();
+  double total = lane < nwarps ? s_part[lane] : 0.0;
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
+  total = __shfl_sync(0xffffffffu, total, 0);
+  const float ms = static_cast<float>(p.inv_cols != 0.0 ? total * p.inv_cols : total / static_cast<double>(p.cols));
+  const float r = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(ms, p.eps)));
+  uint4 n[kSmallChunks];
+  uint32_t amax = 0u;
+  const F32x2 r2 = f32x2(r, r);
+#pragma unroll
+  for (int j = 0; j < kSmallChunks; ++j) {
+    const F32x2 w2[4] = {bf16x2_f32(wv[j].x), bf16x2_f32(wv[j].y), bf16x2_f32(wv[j].z), bf16x2_f32(wv[j].w)};
+    n[j] = norm8(hb[j], r2, w2);
+    amax = amax_acc(amax, n[j]);  // zero past the row's end: w is zero there
+  }
+  uint32_t top;
+  if (CLUSTER) {
+    __shared__ uint32_t s_slots[kMaxClusterCtas];
+    top = cluster_amax_bits(amax, s_amax, s_slots);
+  } else {
+    top = cta_amax_bits(amax, s_amax);
+  }
+  const float tensor_amax = __uint_as_float(top);
+  const Fp8Scale fs = fp8_scale_from_amax(tensor_amax);
+  if (live) {
+#pragma unroll
+    for (int j = 0; j < kSmallChunks; ++j) {
+      const int c = t + j * T;
+      if (c < p.cols8) {
+        reinterpret_cast<uint2*>(p.n_fp8)[row_chunk0 + c] = fp8x8_quant(n[j], fs);
+        if (p.h_out != nullptr) reinterpret_cast<uint4*>(p.h_out)[row_chunk0 + c] = hb[j];
+        if (p.n_bf16 != nullptr) reinterpret_cast<uint4*>(p.n_bf16)[row_chunk0 + c] = n[j];
       }
     }
-    if (blockIdx.x == 0 && t == 0) p.scale_amax[0] = fs.scale, p.scale_amax[1] = tensor_amax;
+    if (t == 0 && p.rstd != nullptr) p.rstd[blockIdx.x] = r;
   }
+  if (blockIdx.x == 0 && t == 0) p.scale_amax[0] = fs.scale, p.scale_amax[1] = tensor_amax;
 }
 
 // The stats sweep for the shape every launch of the Granite sequence has: bf16 y (and res),
@@ -310,16 +390,6 @@ __global__ void __launch_bounds__(256) add_rmsnorm_fast_kernel(const NormParams 
   }
 }
 
-// bf16(h * r * w) of eight packed values, products rounded one after the other.
-__device__ __forceinline__ uint32_t norm_pair(uint32_t h, F32x2 r, F32x2 w) {
-  float a, b;
-  f32x2_split(mul2(mul2(bf16x2_f32(h), r), w), a, b);
-  return pack_bf16x2(a, b);
-}
-__device__ __forceinline__ uint4 norm8(uint4 h, F32x2 r, const F32x2 (&w)[4]) {
-  return make_uint4(norm_pair(h.x, r, w[0]), norm_pair(h.y, r, w[1]), norm_pair(h.z, r, w[2]), norm_pair(h.w, r, w[3]));
-}
-
 // Second sweep with r known per row: a plain streaming pass. A CTA takes kRowsPerCta
 // consecutive rows; a thread takes the chunks t, t + T, ... of each, so every
 // thread has kRowsPerCta * ceil(cols8 / T) independent 128-bit loads to issue
@@ -405,6 +475,13 @@ __global__ void __launch_bounds__(256)
   }
 }
 
+struct QuantSmallParams {
+  const uint4* x;
+  uint2* codes;
+  float* scale_amax;
+  int n8;
+};
+
 // Elementwise per-tensor FP8 of a bf16 tensor: amax sweep, then encode sweep.
 constexpr int kQuantUnroll = 4;
 __global__ void __launch_bounds__(256) amax_bf16_kernel(const uint4* x, long long n8, float* scale_amax) {
@@ -450,34 +527,43 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-// The same for a decode-size tensor (up to 16 rows of 4096): one CTA keeps the tensor in registers,
-// finds max |x| through shared memory and encodes - one launch instead of a memset and two sweeps.
-constexpr int kQuantSmallThreads = 1024, kQuantSmallItems = 8;
+// The same for a decode-size tensor (up to 16 rows of 4096): the tensor stays in the registers of one
+// thread-block cluster of up to eight CTAs (one CTA, no cluster, up to two rows), which finds max |x|
+// and encodes - one launch instead of a memset and two sweeps. Two 16-byte chunks per thread: one CTA
+// for all 16 rows had eight per thread behind one SM's load path: 16 rows 5.2 us, 2.0 now (one row 1.9
+// and 1.1).
+constexpr int kQuantSmallThreads = 512, kQuantSmallItems = 2, kQuantSmallCtas = 8;
+template <bool CLUSTER>
 __global__ void __launch_bounds__(kQuantSmallThreads)
-    quant_small_kernel(const uint4* x, int n8, uint2* codes, float* scale_amax) {
+    quant_small_kernel(const QuantSmallParams p) {
   pdl_begin();
+  if (CLUSTER) cluster_announce();
   __shared__ uint32_t s[kQuantSmallThreads / 32];
+  const int i0 = static_cast<int>(blockIdx.x) * (kQuantSmallThreads * kQuantSmallItems) + threadIdx.x;
   uint4 v[kQuantSmallItems];
   uint32_t amax = 0u;
 #pragma unroll
   for (int k = 0; k < kQuantSmallItems; ++k) {
-    const int i = k * kQuantSmallThreads + threadIdx.x;
-    v[k] = i < n8 ? __ldg(x + i) : make_uint4(0, 0, 0, 0);
-    amax = amax_acc(amax, v[k]);
+    const int i = i0 + k * kQuantSmallThreads;
+    v[k] = i < p.n8 ? __ldg(p.x + i) : make_uint4(0, 0, 0, 0);
   }
-  amax = amax_warp(amax);
-  if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = amax;
-  __syncthreads();
-  uint32_t m = s[threadIdx.x & 31];
-  m = amax_warp(m);
-  const float a = amax_value(m);
+#pragma unroll
+  for (int k = 0; k < kQuantSmallItems; ++k) amax = amax_acc(amax, v[k]);
+  uint32_t top;
+  if (CLUSTER) {
+    __shared__ uint32_t s_slots[kMaxClusterCtas];
+    top = cluster_amax_bits(amax, s, s_slots);
+  } else {
+    top = cta_amax_bits(amax, s);
+  }
+  const float a = __uint_as_float(top);
   const Fp8Scale fs = fp8_scale_from_amax(a);
-  if (threadIdx.x == 0) scale_amax[0] = fs.scale, scale_amax[1] = a;
 #pragma unroll
   for (int k = 0; k < kQuantSmallItems; ++k) {
-    const int i = k * kQuantSmallThreads + threadIdx.x;
-    if (i < n8) codes[i] = fp8x8_quant(v[k], fs);
+    const int i = i0 + k * kQuantSmallThreads;
+    if (i < p.n8) p.codes[i] = fp8x8_quant(v[k], fs);
   }
+  if (blockIdx.x == 0 && threadIdx.x == 0) p.scale_amax[0] = fs.scale, p.scale_amax[1] = a;
 }
 
 int env_int(const char* name, int fallback) {
@@ -541,17 +627,15 @@ int add_rmsnorm_launch(const char* fn, const void* d_y, int y_is_f32, const void
   // the rstd form of the second sweep re-reads h: hold as much of it in L2 as is likely to fit
   p.keep_h = (d_n_fp8 != nullptr && d_n_bf16 == nullptr && d_h_out != nullptr && d_rstd != nullptr)
                  ? l2_keep_fraction(static_cast<double>(rows) * cols * 2.0) : 0.0f;
-  if (d_n_fp8 != nullptr && rows <= kMaxClusterCtas && p.cols8 <= max_threads_for(1) && cluster_enabled()) {
-    const int ctas = cluster_ctas_for(rows);
-    const int threads = (p.cols8 + 31) / 32 * 32;
-    cudaError_t e;
-    if (y_is_f32) {
-      e = res_is_f32 ? cluster_launch(add_rmsnorm_kernel<true, true, 1, kCluster>, ctas, threads, p, st)
-                     : cluster_launch(add_rmsnorm_kernel<true, false, 1, kCluster>, ctas, threads, p, st);
-    } else {
-      e = res_is_f32 ? cluster_launch(add_rmsnorm_kernel<false, true, 1, kCluster>, ctas, threads, p, st)
-                     : cluster_launch(add_rmsnorm_kernel<false, false, 1, kCluster>, ctas, threads, p, st);
-    }
+  if (d_n_fp8 != nullptr && rows <= kMaxClusterCtas && p.cols8 <= 512 * kSmallChunks && cluster_enabled()) {
+    const int threads = ((p.cols8 + kSmallChunks - 1) / kSmallChunks + 31) / 32 * 32;
+    const int kinds = (y_is_f32 ? 1 : 0) | (res_is_f32 ? 2 : 0);
+    void (*const one[4])(NormParams) = {norm_small_kernel<false, false, false>, norm_small_kernel<true, false, false>,
+                                        norm_small_kernel<false, true, false>, norm_small_kernel<true, true, false>};
+    void (*const many[4])(NormParams) = {norm_small_kernel<false, false, true>, norm_small_kernel<true, false, true>,
+                                         norm_small_kernel<false, true, true>, norm_small_kernel<true, true, true>};
+    const cudaError_t e = rows == 1 ? launch_pdl(one[kinds], dim3(1), dim3(static_cast<unsigned>(threads)), 0, st, p)
+                                    : cluster_launch(many[kinds], cluster_ctas_for(rows), threads, p, st);
     if (e == cudaSuccess) return 0;
     if (e != cudaErrorInvalidConfiguration) {
       std::fprintf(stderr, "granite4: %s: cluster launch failed: %s\n", fn, cudaGetErrorString(e));
@@ -672,11 +756,20 @@ int granite4_kernel_fp8_quant(const uint16_t* d_x, long long n, uint8_t* d_codes
   const long long n8 = n / 8;
   const long long grid = g4::quant_grid(n8);
   if (grid > INT_MAX) return g4::fail(fn, "tensor too large");
-  if (n8 <= g4::kQuantSmallThreads * g4::kQuantSmallItems && g4::cluster_enabled()) {  // G4_CLUSTER=0: the two-sweep form
-    G4_LAUNCH_PDL(fn, g4::quant_small_kernel, dim3(1), dim3(g4::kQuantSmallThreads), 0, st,
-                  reinterpret_cast<const uint4*>(d_x), static_cast<int>(n8), reinterpret_cast<uint2*>(d_codes),
-                  d_scale_amax);
-    return 0;
+  constexpr int per_cta = g4::kQuantSmallThreads * g4::kQuantSmallItems;
+  if (n8 <= per_cta * g4::kQuantSmallCtas && g4::cluster_enabled()) {  // G4_CLUSTER=0: the two-sweep form
+    const g4::QuantSmallParams p{reinterpret_cast<const uint4*>(d_x), reinterpret_cast<uint2*>(d_codes), d_scale_amax,
+                                 static_cast<int>(n8)};
+    const cudaError_t e =
+        n8 <= per_cta ? g4::launch_pdl(g4::quant_small_kernel<false>, dim3(1), dim3(g4::kQuantSmallThreads), 0, st, p)
+                      : g4::cluster_launch(g4::quant_small_kernel<true>,
+                                           g4::cluster_ctas_for((n8 + per_cta - 1) / per_cta), g4::kQuantSmallThreads, p, st);
+    if (e == cudaSuccess) return 0;
+    if (e != cudaErrorInvalidConfiguration) {
+      (void)cudaGetLastError();
+      std::fprintf(stderr, "granite4: %s: CUDA error: %s\n", fn, cudaGetErrorString(e));
+      return -1;
+    }
   }
   G4_CUDA_TRY(fn, cudaMemsetAsync(d_scale_amax, 0, 2 * sizeof(float), st));
   G4_LAUNCH_PDL(fn, g4::amax_bf16_kernel, dim3(static_cast<unsigned>(grid)), dim3(256), 0, st,

@@ -43,32 +43,28 @@ __device__ __forceinline__ void cluster_all_started() {
   asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
 }
 
-// Max of `thread_amax` (packed sign-cleared bf16 pairs) over every thread of
-// every CTA in the cluster, as float bits. s_warp: one word per warp of the
-// CTA; s_slots: kMaxClusterCtas words. Called by all threads, in a kernel that
-// began with cluster_announce().
-__device__ __forceinline__ uint32_t cluster_amax_bits(uint32_t thread_amax, uint32_t* s_warp,
-                                                      uint32_t* s_slots) {
+// Max, as float bits, of every thread's packed sign-cleared bf16 pairs over this CTA (NaN stays on top:
+// non-negative floats order as integers). s_warp: one word per warp. Called by all threads.
+__device__ __forceinline__ uint32_t cta_amax_bits(uint32_t thread_amax, uint32_t* s_warp) {
+  const int t = threadIdx.x, warp = t >> 5, lane = t & 31, nwarps = (blockDim.x + 31) >> 5;
+  const uint32_t top = __reduce_max_sync(0xffffffffu, max(thread_amax & 0xffffu, thread_amax >> 16));
+  if (lane == 0) s_warp[warp] = top;
+  __syncthreads();
+  return __reduce_max_sync(0xffffffffu, lane < nwarps ? s_warp[lane] : 0u) << 16;
+}
+
+// The same over every CTA of the cluster, in a kernel that began with cluster_announce(). s_slots:
+// kMaxClusterCtas words.
+__device__ __forceinline__ uint32_t cluster_amax_bits(uint32_t thread_amax, uint32_t* s_warp, uint32_t* s_slots) {
   namespace cg = cooperative_groups;
   cg::cluster_group cluster = cg::this_cluster();
-  const int t = threadIdx.x, warp = t >> 5, lane = t & 31, nwarps = (blockDim.x + 31) >> 5;
-  thread_amax = amax_warp(thread_amax);
-  if (lane == 0) s_warp[warp] = thread_amax;
-  __syncthreads();
+  const uint32_t mine = cta_amax_bits(thread_amax, s_warp);
   cluster_all_started();  // pairs with the cluster_announce() at the top of the calling kernel
-  const unsigned n = cluster.num_blocks();
-  if (warp == 0) {
-    uint32_t m = 0u;
-    for (int i = lane; i < nwarps; i += 32) m = max_u16x2(m, s_warp[i]);
-    m = amax_warp(m);
-    // lane d delivers this CTA's maximum into CTA d's slot for this CTA
-    if (static_cast<unsigned>(lane) < n)
-      *cluster.map_shared_rank(s_slots + cluster.block_rank(), lane) = __float_as_uint(amax_value(m));
-  }
+  const unsigned n = cluster.num_blocks(), lane = threadIdx.x & 31u;
+  // thread d delivers this CTA's maximum into CTA d's slot for this CTA
+  if (threadIdx.x < n) *cluster.map_shared_rank(s_slots + cluster.block_rank(), threadIdx.x) = mine;
   cluster.sync();  // release / acquire: the remote stores above are visible after it
-  uint32_t g = 0u;
-  for (unsigned i = 0; i < n; ++i) g = max(g, s_slots[i]);  // non-negative floats order as integers; NaN stays on top
-  return g;
+  return __reduce_max_sync(0xffffffffu, lane < n ? s_slots[lane] : 0u);
 }
 
 // G4_CLUSTER=0 in the environment keeps every op on its multi-launch form (A/B runs, tests that

@@ -325,6 +325,10 @@ __device__ __forceinline__ float4 ld_stream(const float4* p) { return __ldcs(p);
 __device__ __forceinline__ void st_stream(uint4* p, uint4 v) { __stcs(p, v); }
 __device__ __forceinline__ void st_stream(uint2* p, uint2 v) { __stcs(p, v); }
 
+// Asks the line of `p` into L2. Reads nothing, so it may be issued before griddepcontrol.wait even for
+// memory the kernel ahead might still write.
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
 // L2 eviction-priority hints on single loads and stores (an instruction-level policy operand;
 // nothing about the device or the context is configured). A tensor that one sweep writes and the
 // next sweep re-reads is stored with evict_last so that the read-once inputs streaming past it do

@@ -73,32 +73,31 @@ struct RopeKvParams {
 constexpr int kD = 128;
 constexpr int kHeadsPerCta = 16;
 
-// One 128-thread CTA handles kRows token rows, all heads: thread (g, j) = (tid / 8, tid % 8) owns
-// lane j of the heads g, g + 16, g + 32, ... of each row. The cos / sin values of lane j depend
-// only on the row, so they are loaded once per row and reused for every head of the thread.
-// All the activation loads of a row are issued before the first is used.
+// Thread (g, j) = (tid / 8, tid % 8) of a 128-thread CTA owns lane j of the heads g + 16 b, with b =
+// blockIdx.y, blockIdx.y + gridDim.y, ... of token row blockIdx.x: one head per thread when gridDim.y
+// covers the heads, all of a row's heads in one CTA when it is 1. The cos / sin values of lane j depend
+// only on the row, so they are loaded once and reused for every head of the thread. The activation
+// loads are issued before the row's position is known: a decode step is one chain of dependent loads
+// (position -> table row), and everything else overlaps it. 1 - 16 rows: 2.3 us, against 3.1 for the staged
+// form below; at 500 and 777 rows the two forms measured the same.
 constexpr int kMaxHeadsPerThread = 4;  // (Hq + 2 Hk) <= 64 heads per row in this kernel
 
-template <int kRows>
 __global__ void __launch_bounds__(kHeadsPerCta * 8) rope_kv_int8_kernel(const RopeKvParams p) {
   pdl_begin();
-  const int g = threadIdx.x >> 3;
+  const int g = (threadIdx.x >> 3) + blockIdx.y * kHeadsPerCta;
+  const int step = gridDim.y * kHeadsPerCta;
   const int j = threadIdx.x & 7;
   const int heads_total = p.Hq + 2 * p.Hk;
   const unsigned gmask = 0xffu << (threadIdx.x & 24);  // the 8 lanes that share this thread's heads
-#pragma unroll
-  for (int i = 0; i < kRows; ++i) {
-    const int r = blockIdx.x * kRows + i;
-    if (r >= p.rows) return;  // uniform over the CTA
+  {
+    const int r = blockIdx.x;
     int pos, kv_row;
-    if (p.mode == kRunOfPositions) {
-      pos = p.base_pos + r;
-      kv_row = p.d_pt != nullptr ? __ldg(p.d_pt + pos) : pos;
-    } else if (p.mode == kPerRowArrays) {
+    if (p.mode == kPerRowArrays) {
       pos = __ldg(p.pos_rows + r);
       kv_row = __ldg(p.kv_rows + r);
-      // a bad index skips the row instead of touching memory outside the tables or the pool
-      if (pos < 0 || pos >= p.max_pos || kv_row < 0 || kv_row >= p.stride) continue;
+    } else if (p.mode == kRunOfPositions) {
+      pos = p.base_pos + r;
+      kv_row = p.d_pt != nullptr ? __ldg(p.d_pt + pos) : pos;
     } else {
       pos = p.mr->pos[r];
       const int slot = p.mr->tree ? p.mr->slot[r] : pos;
@@ -108,7 +107,7 @@ __global__ void __launch_bounds__(kHeadsPerCta * 8) rope_kv_int8_kernel(const Ro
     uint4 xlo[kMaxHeadsPerThread], xhi[kMaxHeadsPerThread];
 #pragma unroll
     for (int k = 0; k < kMaxHeadsPerThread; ++k) {
-      const int head = g + k * kHeadsPerCta;
+      const int head = g + k * step;
       if (head >= heads_total) break;
       const uint16_t* src;
       if (head < p.Hq) src = p.q + static_cast<size_t>(r) * p.pitch_q + static_cast<size_t>(head) * kD;
@@ -117,6 +116,8 @@ __global__ void __launch_bounds__(kHeadsPerCta * 8) rope_kv_int8_kernel(const Ro
       xlo[k] = ld_stream(reinterpret_cast<const uint4*>(src) + j);
       xhi[k] = ld_stream(reinterpret_cast<const uint4*>(src) + 8 + j);
     }
+    // a bad index skips the row instead of touching memory outside the tables or the pool
+    if (p.mode == kPerRowArrays && (pos < 0 || pos >= p.max_pos || kv_row < 0 || kv_row >= p.stride)) return;
     float c[8], s[8];
     if (p.cos_tbl != nullptr) {
       const float4* cp = reinterpret_cast<const float4*>(p.cos_tbl + static_cast<size_t>(pos) * (kD / 2)) + 2 * j;
@@ -130,7 +131,7 @@ __global__ void __launch_bounds__(kHeadsPerCta * 8) rope_kv_int8_kernel(const Ro
     }
 #pragma unroll
     for (int k = 0; k < kMaxHeadsPerThread; ++k) {
-      const int head = g + k * kHeadsPerCta;
+      const int head = g + k * step;
       if (head >= heads_total) break;
       const bool is_q = head < p.Hq;
       const bool is_k = !is_q && head < p.Hq + p.Hk;
@@ -428,13 +429,15 @@ __global__ void __launch_bounds__(1024)
   cache_v[srow * d + i] = static_cast<int8_t>(kv8_quant_exact(y, sv));
 }
 
+// Up to this many rows (a decode or verify step): a CTA per row and 16 heads, no staging.
+constexpr int kSplitHeadsRows = 16;
 int launch_rope_kv(const char* fn, RopeKvParams& p) {
   const int heads_total = p.Hq + 2 * p.Hk;
   if (heads_total > kMaxHeadsPerThread * kHeadsPerCta) return fail(fn, "more than 64 heads per row");
   cudaStream_t st = current_stream();
   // Bulk-copy path (default): needs 16-byte aligned sources and a status word to report to.
   const char* env = std::getenv("G4_ROPE_BULK");
-  const bool want_bulk = !(env != nullptr && env[0] == '0');
+  const bool want_bulk = !(env != nullptr && env[0] == '0') && p.rows > kSplitHeadsRows;
   unsigned int* status = want_bulk ? device_status_ptr() : nullptr;
   const size_t stage_bytes = static_cast<size_t>(heads_total) * kD * 2 + 2 * (kD / 2) * 4;
   const size_t smem = kBulkStages * stage_bytes + kBulkStages * (2 * sizeof(uint64_t) + sizeof(RowMeta)) + 16;
@@ -454,8 +457,8 @@ int launch_rope_kv(const char* fn, RopeKvParams& p) {
     const unsigned grid = static_cast<unsigned>(std::min<long long>(p.rows, static_cast<long long>(sm_count()) * per_sm));
     G4_LAUNCH_PDL(fn, rope_kv_bulk_kernel, dim3(grid), dim3(kBulkThreads), smem, st, p, status);
   } else {
-    G4_LAUNCH_PDL(fn, rope_kv_int8_kernel<1>, dim3(static_cast<unsigned>(p.rows)), dim3(kHeadsPerCta * 8), 0,
-                  st, p);
+    const unsigned parts = p.rows <= kSplitHeadsRows ? static_cast<unsigned>((heads_total + kHeadsPerCta - 1) / kHeadsPerCta) : 1u;
+    G4_LAUNCH_PDL(fn, rope_kv_int8_kernel, dim3(static_cast<unsigned>(p.rows), parts), dim3(kHeadsPerCta * 8), 0, st, p);
   }
   return 0;
 }

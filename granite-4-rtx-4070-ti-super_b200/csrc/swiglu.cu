@@ -155,20 +155,22 @@ __global__ void __launch_bounds__(kThreads) swiglu_kernel(const SwigluParams p) 
 
 // Small tensors (a decode or verify step: up to 16 rows of 12800): the whole grid is one cluster,
 // the activations stay in registers between the amax exchange and the encode step, so one launch
-// replaces the memset and the two sweeps (g4_cluster.cuh). A CTA owns kClusterThreads * kUnroll
-// consecutive items.
+// replaces the memset and the two sweeps (g4_cluster.cuh). One row is 25 600 special-function
+// instructions, 0.85 us on one SM, so the items are spread: one per thread while 16 CTAs of 512 threads
+// last (five rows), up to kUnroll beyond. A CTA owns UN * kClusterThreads consecutive items.
+// One row: 4.6 us with all its items on one CTA, 2.2 now.
 constexpr int kClusterThreads = 512;
-constexpr long long kClusterItemsPerCta = static_cast<long long>(kClusterThreads) * kUnroll;
+constexpr long long kClusterItemsMax = static_cast<long long>(kMaxClusterCtas) * kClusterThreads * kUnroll;
 
-template <bool F32>
+template <bool F32, int UN>
 __global__ void __launch_bounds__(kClusterThreads) swiglu_cluster_kernel(const SwigluParams p) {
   pdl_begin();
   cluster_announce();
-  const long long tile0 = static_cast<long long>(blockIdx.x) * kClusterItemsPerCta + threadIdx.x;
-  uint4 a[kUnroll];
+  const long long tile0 = static_cast<long long>(blockIdx.x) * (kClusterThreads * UN) + threadIdx.x;
+  uint4 a[UN];
   uint32_t amax = 0u;
 #pragma unroll
-  for (int k = 0; k < kUnroll; ++k) {
+  for (int k = 0; k < UN; ++k) {
     const long long it = tile0 + k * kClusterThreads;
     a[k] = make_uint4(0, 0, 0, 0);
     if (it < p.items) {
@@ -182,9 +184,9 @@ __global__ void __launch_bounds__(kClusterThreads) swiglu_cluster_kernel(const S
   const float tensor_amax = __uint_as_float(cluster_amax_bits(amax, s_warp, s_slots));
   const Fp8Scale fs = fp8_scale_from_amax(tensor_amax);
 #pragma unroll
-  for (int k = 0; k < kUnroll; ++k) {
+  for (int k = 0; k < UN; ++k) {
     const long long it = tile0 + k * kClusterThreads;
-    if (it < p.items) st_stream(reinterpret_cast<uint2*>(p.act_fp8) + it, fp8x8_quant(a[k], fs));
+    if (it < p.items) reinterpret_cast<uint2*>(p.act_fp8)[it] = fp8x8_quant(a[k], fs);
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) p.scale_amax[0] = fs.scale, p.scale_amax[1] = tensor_amax;
 }
@@ -208,9 +210,14 @@ int launch_swiglu(const char* fn, const SwigluParams& p) {
     G4_LAUNCH_PDL(fn, swiglu_kernel<F32, kPlain, false>, dim3(grid), dim3(kThreads), 0, st, p);
     return 0;
   }
-  if (p.items <= kMaxClusterCtas * kClusterItemsPerCta && cluster_enabled()) {
-    const int ctas = cluster_ctas_for((p.items + kClusterItemsPerCta - 1) / kClusterItemsPerCta);
-    const cudaError_t e = cluster_launch(swiglu_cluster_kernel<F32>, ctas, kClusterThreads, p, st);
+  if (p.items <= kClusterItemsMax && cluster_enabled()) {
+    const long long blocks = (p.items + kClusterThreads - 1) / kClusterThreads;
+    const cudaError_t e =
+        blocks <= kMaxClusterCtas
+            ? cluster_launch(swiglu_cluster_kernel<F32, 1>, cluster_ctas_for(blocks), kClusterThreads, p, st)
+        : blocks <= 2 * kMaxClusterCtas
+            ? cluster_launch(swiglu_cluster_kernel<F32, 2>, kMaxClusterCtas, kClusterThreads, p, st)
+            : cluster_launch(swiglu_cluster_kernel<F32, kUnroll>, kMaxClusterCtas, kClusterThreads, p, st);
     if (e == cudaSuccess) return 0;
     if (e != cudaErrorInvalidConfiguration) {
       std::fprintf(stderr, "granite4: %s: cluster launch failed: %s\n", fn, cudaGetErrorString(e));
