@@ -39,6 +39,14 @@ __device__ __forceinline__ void mma_commit(uint32_t bar) {
   else
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
+// The pair form of the same, signalling the barrier at this offset in BOTH CTAs of the cluster: the peer
+// learns of the completion without a relay through the leader.
+__device__ __forceinline__ void mma_commit_both(uint32_t bar) {
+  asm volatile(
+      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar),
+      "h"(uint16_t(3))
+      : "memory");
+}
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
@@ -61,6 +69,21 @@ __device__ __forceinline__ uint32_t cluster_rank() {
 __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+// One lane of a converged warp, the same one every time. A loop that issues MMAs is best run by the whole
+// warp with only the MMAs and commits under this predicate: their descriptors then stay in uniform
+// registers. Under `if (lane == 0)` each MMA waits for its operands to be moved there: 72 cycles per MMA
+// whatever its size, against 43 - 57 (measured, M 128 / pair M 256, up to 96 columns).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t e;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(e));
+  return e != 0u;
+}
+// Index of the warp in its CTA, as a value the compiler knows to be the same in every lane.
+__device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, int(threadIdx.x) >> 5, 0); }
 // 32 lanes x 32 consecutive 32-bit columns: thread t of the warp gets lane (base lane + t).
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
   asm volatile(

@@ -15,15 +15,17 @@
 // rows, the 16-row form with split K and the fused SwiGLU epilogue are described
 // at Cfg, plan_split and store_accumulator_swiglu): persistent, one CTA per SM,
 // 128 x 256 output tiles, K consumed in 128-byte blocks. Roles by warp:
-//   warp 0   one thread issues the tiled TMA loads (128-byte swizzle) of the A
-//            and W blocks into a 4-stage shared-memory ring;
-//   warp 1   allocates tensor memory; one thread issues tcgen05.mma
+//   warps 0, 7 and 6, 8  one thread each issues the tiled TMA loads (128-byte
+//            swizzle) of the W and A blocks, k-blocks in turn, into a
+//            shared-memory ring;
+//   warp 1   allocates tensor memory; one lane issues tcgen05.mma
 //            (kind::f8f6f4, M 128, N 256, K 32 per instruction) straight from
 //            the ring into one of two 256-column accumulators, and commits each
-//            stage back to the loader and each finished tile to the epilogue;
+//            stage back to the loaders and each finished tile to the epilogue;
 //   warps 2-5 read the finished accumulator out of tensor memory (each warp its
-//            own 32 lanes = 32 output rows), scale, convert and store, while
-//            the next tile's MMAs fill the other accumulator.
+//            own 32 lanes = 32 output rows), scale, convert and store through
+//            shared memory by TMA, while the next tile's MMAs fill the other
+//            accumulator.
 // Every wait on an mbarrier is bounded; a wait that runs out sets the library's
 // device status word and an abort flag that winds all roles down, after which
 // the CTA waits a bounded time for copies in flight and frees its tensor memory.
@@ -48,10 +50,15 @@ using namespace g4;
 
 constexpr int kBM = 128, kBN = 256, kBK = 128;  // kBK in bytes = e4m3 elements
 constexpr int kAccs = 2;
-constexpr int kThreads = 192;
+constexpr int kThreads = 192;        // stream form: loader, MMA, four epilogue warps
+constexpr int kTileThreads = 288;    // tiled forms: W loader, MMA, four epilogue warps, A loader, second W and A loaders
 constexpr uint32_t kTmemCols = kAccs * kBN;  // 512: the whole tensor memory of the SM
-constexpr int kMaxStages = 6;
+constexpr int kMaxStages = 9;
 constexpr int kMaxSplits = 16;
+
+// Output (and residual) tiles pass through shared memory in slabs of 32 rows x 128 bytes, two per
+// epilogue warp, and move by TMA: see store_slabs.
+constexpr uint32_t kSlabBytes = 32 * 128, kEpiBytes = 4 * 2 * kSlabBytes;
 
 // Forms of the kernel; all compute 256 output columns per tile: a stage costs the loader thread
 // about 0.3 us of issue (barrier wait, expect_tx, two TMA instructions) whatever its size, so only
@@ -72,10 +79,12 @@ struct Cfg {
   static constexpr uint32_t kABytes = kARows * kBK, kWBytes = kWRows * kBK;
   static constexpr uint32_t kStageBytes = kABytes + kWBytes;
   static constexpr int kTileM = kPair ? 2 * kBM : kBM;
-  // the MMA reads kBM rows of A wherever kARows ends: keep that inside the allocation
-  static constexpr size_t kSmemBytes = 1024 + size_t(kStages) * kStageBytes + (kBM - kARows) * kBK + 256;
-  // Instruction descriptor: f32 accumulator, e4m3 x e4m3, both operands K-major, N 256, M 128 / 256.
-  static constexpr uint32_t kIdesc = (1u << 4) | (uint32_t(kBN >> 3) << 17) | (uint32_t(kTileM >> 4) << 24);
+  // the epilogue's slabs behind the ring; the MMA reads kBM rows of A wherever kARows ends: keep that
+  // inside the allocation
+  static constexpr uint32_t kEpiOffset = uint32_t(kStages) * kStageBytes + ((kBM - kARows) * kBK + 1023) / 1024 * 1024;
+  static constexpr size_t kSmemBytes = 1024 + size_t(kEpiOffset) + kEpiBytes + 256;
+  // Instruction descriptor: f32 accumulator, e4m3 x e4m3, both operands K-major, M 128 / 256; N added at run time.
+  static constexpr uint32_t kIdescM = (1u << 4) | (uint32_t(kTileM >> 4) << 24);
   static_assert(kStages <= kMaxStages && kSmemBytes <= 227 * 1024, "ring too large");
   static_assert(!kPair || kARows == kBM, "the pair form loads whole A blocks");
 };
@@ -85,6 +94,7 @@ using CfgSkinny = Cfg<false, 16, 5>;
 
 struct Ring {
   uint64_t full[kMaxStages], empty[kMaxStages], acc_full[kAccs], acc_empty[kAccs];
+  uint64_t res_full[4][2];  // residual slabs, per epilogue warp and buffer
   uint32_t tmem_base;
   int abort;
   int last;  // split K: whether this CTA delivered the last partial of the current tile
@@ -104,7 +114,7 @@ struct GemmParams {
   int splits, kb_per, ws_rows;
   int early;  // decode-size launch: see the dependent-launch note in the kernel
   // stream form (gemm_fp8_stream_kernel): tile columns, k blocks per stage, rows of A fetched, ring depth
-  int bn, kc, a_rows, stages;
+  int bn, kc, a_rows, stages;  // (bn: also the tile columns of the pair form)
   int box3d;  // one TMA box spans the kc k-blocks of a stage (needs K % 128 == 0)
   // fused SwiGLU (out_kind SWIGLU): W is gate rows [0, I) then up rows [I, 2 I); a tile is 128 output
   // columns whose accumulator holds gate in columns 0..127 and up in 128..255
@@ -266,21 +276,21 @@ __device__ __forceinline__ void store4(const GemmParams& p, float4 v, int row, i
   }
 }
 
-// Fused SwiGLU epilogue of one warp's 32 rows: gate from columns 0..127 and up from columns 128..255 of
-// the accumulator, a = bf16(silu(g) u) (the arithmetic of the standalone kernel, g4_math.cuh swiglu) for
-// output columns n0 .. n0 + 127, and the running max |a| of what was stored (packed bf16 pairs).
+// Fused SwiGLU epilogue of one warp's 32 rows: gate from the first `half` columns of the accumulator and
+// up from the next, a = bf16(silu(g) u) (the arithmetic of the standalone kernel, g4_math.cuh swiglu) for
+// output columns n0 .. n0 + half - 1, and the running max |a| of what was stored (packed bf16 pairs).
 __device__ __forceinline__ uint32_t store_accumulator_swiglu(const GemmParams& p, uint32_t taddr, int row, int n0,
-                                                             float a_scale) {
+                                                             float a_scale, int half) {
   uint32_t amax = 0u;
   const int I = p.swiglu_i;
 #pragma unroll 1
-  for (int c = 0; c < 4; ++c) {
+  for (int c = 0; c < half / 32; ++c) {
     const int n = n0 + c * 32;
     if (n >= I) break;  // uniform over the warp
     uint32_t gv[32], uv[32];
     __syncwarp();
     tmem_ld32(taddr + c * 32, gv);
-    tmem_ld32(taddr + 128 + c * 32, uv);
+    tmem_ld32(taddr + half + c * 32, uv);
     tmem_ld_wait();
     if (row >= p.M) continue;
     const bool one_scale = (n >= p.seg1 || n + 32 <= p.seg1) && (n >= p.seg2 || n + 32 <= p.seg2) &&
@@ -316,10 +326,10 @@ __device__ __forceinline__ uint32_t store_accumulator_swiglu(const GemmParams& p
 // One warp's 32 rows x 256 columns of a finished accumulator: tensor memory -> epilogue -> global,
 // or (partial != NULL, split K) tensor memory -> this unit's f32 partial rows [.][256].
 // Every lane executes the tensor-memory loads; lanes past row M skip the stores.
-__device__ __forceinline__ void store_accumulator(const GemmParams& p, uint32_t taddr, int row, int n0, float a_scale,
-                                                  float* partial_row) {
+__device__ __forceinline__ void store_accumulator(const GemmParams& p, uint32_t taddr, int row, int n0, int cols,
+                                                  float a_scale, float* partial_row) {
 #pragma unroll 1
-  for (int c = 0; c < kBN / 32; ++c) {
+  for (int c = 0; c < cols / 32; ++c) {
     const int n = n0 + c * 32;
     if (n >= p.N) break;  // uniform over the warp
     uint32_t v[32];
@@ -335,31 +345,179 @@ __device__ __forceinline__ void store_accumulator(const GemmParams& p, uint32_t 
       float f[32];
 #pragma unroll
       for (int j = 0; j < 32; ++j) f[j] = __uint_as_float(v[j]);
-      store_chunk(p, f, row, n, a_scale, p.N);
+      store_chunk(p, f, row, n, a_scale, min(p.N, n0 + cols));
     }
   }
 }
 
+// ---- epilogue through shared memory --------------------------------------------------------------
+// A thread holds one output ROW of the accumulator, so storing from registers writes 16 bytes to each of
+// 32 rows per instruction: 1.2 us per 32 columns of a 128-row tile, 9.5 us for a 256-column one, which a
+// launch of one tile per CTA pays in full. Here a warp writes its 32 rows into a slab of shared memory
+// (32 rows x 128 bytes, 128-byte swizzle: conflict-free) and one TMA store per slab sends it on while the
+// next is computed; ragged edges are the tensor map's. A residual comes the same way, by TMA into the slab
+// that its sum then replaces, two slabs ahead. QKV of 500 rows 24.4 -> 17.8 us, of 8192 rows 176 -> 144 us;
+// O with the residual (eight dependent loads per row before) of 8192 rows 206 -> 101 us.
+__device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, uint32_t src, int x, int y) {
+  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%1, %2}], [%3];" ::"l"(
+                   reinterpret_cast<uint64_t>(map)),
+               "r"(x), "r"(y), "r"(src)
+               : "memory");
+}
+__device__ __forceinline__ uint32_t slab_at(uint32_t slab, int row, int chunk) {
+  return slab + uint32_t(row * 128 + ((chunk ^ (row & 7)) << 4));
+}
+__device__ __forceinline__ void slab_put(uint32_t addr, uint4 v) {
+  asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+}
+__device__ __forceinline__ uint4 slab_get(uint32_t addr) {
+  uint4 v;
+  asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
+  return v;
+}
+
+// One epilogue warp's buffers. `count` slabs have gone through them so far.
+struct SlabState {
+  uint32_t base;      // shared-memory address of its two slabs
+  uint64_t* res_full;  // [2]
+  uint32_t count;
+};
+
+__device__ __forceinline__ void residual_slab(const CUtensorMap* map_res, const SlabState& st, uint32_t index, int x, int y) {
+  uint64_t* bar = st.res_full + (index & 1u);
+  mbar_arrive_expect_tx(bar, kSlabBytes);
+  tma_load_2d<false>(st.base + (index & 1u) * kSlabBytes, map_res, x, y, smem_u32(bar));
+}
+// Lane 0, before a tile's accumulator is complete: the first two residual slabs of the warp's rows.
+__device__ __forceinline__ void residual_ahead(const CUtensorMap* map_res, const SlabState& st, int n0, int n_end, int row0) {
+  bulk_wait_read<0>();  // the last tile's stores have read their slabs
+  residual_slab(map_res, st, st.count, n0, row0);
+  if (n0 + 64 < n_end) residual_slab(map_res, st, st.count + 1, n0 + 64, row0);
+}
+
+// Columns n0 .. n_end - 1 of rows row0 .. row0 + 31 (row0 < M; n0 < n_end <= N) from the accumulator at
+// taddr. Returns the running max |.| of the fused SwiGLU's outputs (packed bf16 pairs; of stored elements
+// only: rows and columns past the output are zero in the accumulator). ok: false once a wait ran out.
+__device__ __forceinline__ uint32_t store_slabs(const GemmParams& p, const CUtensorMap* map_out, const CUtensorMap* map_res,
+                                                SlabState& st, Ring* ring, uint32_t taddr, int lane, int row0, int n0,
+                                                int n_end, int half, float a_scale, bool& ok) {
+  uint32_t amax = 0u;
+  const bool f32 = p.out_kind == GRANITE4_GEMM_OUT_F32, resid = p.out_kind == GRANITE4_GEMM_OUT_RESIDUAL;
+  const int width = f32 ? 32 : 64;
+#pragma unroll 1
+  for (int n = n0; n < n_end; n += width, ++st.count) {
+    const uint32_t slab = st.base + (st.count & 1u) * kSlabBytes;
+    if (resid) {
+      if (!wait_or_abort(st.res_full + (st.count & 1u), (st.count >> 1) & 1u, ring, p.status)) {
+        ok = false;
+        break;
+      }
+    } else {
+      if (lane == 0) bulk_wait_read<1>();  // the store from this slab two steps ago has read it
+    }
+    __syncwarp();
+#pragma unroll 1
+    for (int h = 0; h < width / 32; ++h) {
+      const int nc = n + h * 32;
+      uint32_t v[32];
+      tmem_ld32(taddr + (nc - n0), v);
+      if (p.swiglu_i) {
+        const int I = p.swiglu_i;
+        uint32_t u[32];
+        tmem_ld32(taddr + half + (nc - n0), u);
+        tmem_ld_wait();
+        const bool one = (nc >= p.seg1 || nc + 32 <= p.seg1) && (nc >= p.seg2 || nc + 32 <= p.seg2) &&
+                         (I + nc >= p.seg1 || I + nc + 32 <= p.seg1) && (I + nc >= p.seg2 || I + nc + 32 <= p.seg2);
+        const float sg = a_scale * seg_scale(p, nc), su = a_scale * seg_scale(p, I + nc);
+        float a[32];
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
+          float g = __fmul_rn(sg, __uint_as_float(v[j])), x = __fmul_rn(su, __uint_as_float(u[j]));
+          if (!one)
+            g = __fmul_rn(a_scale * seg_scale(p, nc + j), __uint_as_float(v[j])), x = __fmul_rn(a_scale * seg_scale(p, I + nc + j), __uint_as_float(u[j]));
+          a[j] = swiglu(g, x);
+        }
+        // columns past I: the accumulator's gate and up columns belong to other rows of W there
+        if (nc + 32 > I) {
+#pragma unroll
+          for (int j = 0; j < 32; ++j)
+            if (nc + j >= I) a[j] = 0.0f;
+        }
+#pragma unroll
+        for (int j = 0; j < 32; j += 8) {
+          const uint4 w = make_uint4(pack_bf16x2(a[j], a[j + 1]), pack_bf16x2(a[j + 2], a[j + 3]), pack_bf16x2(a[j + 4], a[j + 5]),
+                                     pack_bf16x2(a[j + 6], a[j + 7]));
+          amax = amax_acc(amax, w);
+          slab_put(slab_at(slab, lane, h * 4 + j / 8), w);
+        }
+        continue;
+      }
+      tmem_ld_wait();
+      const bool one = (nc >= p.seg1 || nc + 32 <= p.seg1) && (nc >= p.seg2 || nc + 32 <= p.seg2);
+      const float sc = a_scale * seg_scale(p, nc);
+      float y[32];
+#pragma unroll
+      for (int j = 0; j < 32; ++j) y[j] = sc * __uint_as_float(v[j]);
+      if (!one) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) y[j] = (a_scale * seg_scale(p, nc + j)) * __uint_as_float(v[j]);
+      }
+      if (f32) {
+#pragma unroll
+        for (int j = 0; j < 32; j += 4)
+          slab_put(slab_at(slab, lane, j / 4), make_uint4(__float_as_uint(y[j]), __float_as_uint(y[j + 1]), __float_as_uint(y[j + 2]), __float_as_uint(y[j + 3])));
+        continue;
+      }
+#pragma unroll
+      for (int j = 0; j < 32; j += 8) {
+        const uint32_t at = slab_at(slab, lane, h * 4 + j / 8);
+        if (resid) {
+          float r[8];
+          unpack8(slab_get(at), r);
+#pragma unroll
+          for (int e = 0; e < 8; ++e) y[j + e] = __fadd_rn(r[e], __fmul_rn(p.resid_scale, y[j + e]));
+        }
+        slab_put(at, make_uint4(pack_bf16x2(y[j], y[j + 1]), pack_bf16x2(y[j + 2], y[j + 3]), pack_bf16x2(y[j + 4], y[j + 5]),
+                                pack_bf16x2(y[j + 6], y[j + 7])));
+      }
+    }
+    fence_async_smem();  // the slab is read by the copy engine
+    __syncwarp();
+    if (lane == 0) {
+      // the residual slab after the next takes the buffer of the store before this one
+      if (resid && n > n0 && n + width < n_end) {
+        bulk_wait_read<0>();
+        residual_slab(map_res, st, st.count + 1, n + width, row0);
+      }
+      tma_store_2d(map_out, slab, n, row0);
+      bulk_commit();
+    }
+  }
+  return amax;
+}
+
 template <class C>
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(kTileThreads, 1)
 gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
-                const GemmParams p) {
+                const __grid_constant__ CUtensorMap map_out, const __grid_constant__ CUtensorMap map_res, const GemmParams p) {
   constexpr bool kPair = C::kTileM == 2 * kBM;
   constexpr uint32_t kABytes = C::kABytes;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t tiles_addr = (raw + 1023u) & ~1023u;  // swizzled tiles sit on 1024-byte boundaries
   uint8_t* tiles_ptr = smem_raw + (tiles_addr - raw);
-  Ring* ring = reinterpret_cast<Ring*>(tiles_ptr + size_t(C::kStages) * C::kStageBytes);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  Ring* ring = reinterpret_cast<Ring*>(tiles_ptr + C::kEpiOffset + kEpiBytes);
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const uint32_t rank = kPair ? cluster_rank() : 0u;  // CTA of the pair; 0 leads
   const bool leader = rank == 0u;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < C::kStages; ++s) mbar_init(&ring->full[s], 1), mbar_init(&ring->empty[s], 1);
+    // a stage is armed by the (leader's) W loader and A loader, each for its own bytes
+    for (int s = 0; s < kMaxStages; ++s) mbar_init(&ring->full[s], 2), mbar_init(&ring->empty[s], 1);
     // a finished accumulator is released by the four epilogue warps of every CTA that reads it;
-    // in the pair form only the leader's barriers of this kind are waited on
+    // in the pair form only the leader's acc_empty is waited on
     for (int a = 0; a < kAccs; ++a) mbar_init(&ring->acc_full[a], 1), mbar_init(&ring->acc_empty[a], kPair ? 8 : 4);
+    for (int w = 0; w < 4; ++w) mbar_init(&ring->res_full[w][0], 1), mbar_init(&ring->res_full[w][1], 1);
     ring->abort = 0;
     mbar_init_fence();
     fence_async_smem();
@@ -372,77 +530,68 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
   const uint32_t tmem_base = ring->tmem_base;
 
   // Programmatic dependent launch. Everything above touches no global memory. The weights are
-  // constants of the model, not products of the kernel before this one on the stream, so the
-  // loader thread of the decode-size forms (p.early) fetches the first stages' W blocks before it
-  // waits for that kernel; whatever reads activations, residuals, scales or the workspace, and
-  // everything that writes, comes after the wait. Those forms also let the kernel after them
-  // start as soon as CTAs of this one retire: with a few microseconds of work per launch, the
-  // ramps of consecutive GEMMs are most of the time otherwise.
-  const bool loader = warp == 0 && lane == 0;
+  // constants of the model, not products of the kernel before this one on the stream, so the W
+  // loader does not wait for that kernel; whatever reads activations, residuals, scales or the
+  // workspace, and everything that writes, comes after the wait. The decode-size forms (p.early) also
+  // let the kernel after them start as soon as CTAs of this one retire: with a few microseconds of
+  // work per launch, the ramps of consecutive GEMMs are most of the time otherwise.
   if (p.early) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  if (!(loader && p.early)) pdl_begin();
+  if (warp != 0 && warp != 7) asm volatile("griddepcontrol.wait;" ::: "memory");
 
-  const int tile_cols = p.swiglu_i ? kBN / 2 : kBN;  // output columns of a tile
+  const int bn = kPair ? p.bn : kBN;                  // accumulator columns of a tile
+  const int tile_cols = p.swiglu_i ? bn / 2 : bn;     // output columns of a tile
+  const uint32_t w_bytes = uint32_t(kPair ? bn / 2 : bn) * kBK;
+  // narrower tiles make smaller stages, and more of them in the same ring
+  const uint32_t stage_bytes = kABytes + w_bytes;
+  const uint32_t stages = kPair ? min(uint32_t(kMaxStages), uint32_t(C::kStages) * uint32_t(C::kStageBytes) / stage_bytes) : uint32_t(C::kStages);
   const int mt = (p.M + C::kTileM - 1) / C::kTileM, nt = ((p.swiglu_i ? p.swiglu_i : p.N) + tile_cols - 1) / tile_cols;
   const int tiles = mt * nt, kblocks = (p.K + kBK - 1) / kBK;
   const int units = tiles * p.splits;  // splits == 1 unless K is split
   const int first = kPair ? int(blockIdx.x >> 1) : int(blockIdx.x);
   const int step = kPair ? int(gridDim.x >> 1) : int(gridDim.x);
 
-  if (warp == 0) {
+  if (warp == 0 || warp >= 6) {
     if (lane == 0) {
+      // Two threads per operand: a thread gets through one tiled copy per 0.2 - 0.3 us (ring wait, expect_tx,
+      // issue), and a k-block of a 64-column tile is 0.16 us.
       // Pair form: both CTAs load their own halves; every completion is counted on the leader's
-      // `full` barrier, which the leader arms for both halves. The peer may refill a stage when
-      // the leader has seen the MMAs that read it complete, which the leader passes on.
+      // `full` barrier, which the leader's loaders arm for both halves (bytes that arrive before they are
+      // announced only make the count negative for a moment). The commit of the MMAs that read a stage
+      // frees it in both CTAs at once; relayed by the leader's loader, the round trip of a stage was
+      // ~2 us.
+      const bool is_a = warp == 6 || warp == 8;
+      uint32_t turn = warp >= 7 ? 1u : 0u;  // 0: this k-block is this thread's, 1: the other's
       const uint32_t full0 = kPair ? cluster_addr(smem_u32(&ring->full[0]), 0) : smem_u32(&ring->full[0]);
-      uint32_t it = 0, ahead = 0;  // ahead: stages whose W block was fetched before the dependency wait
-      if (!kPair && p.early) {
-        for (int u = first; u < units && ahead < uint32_t(C::kStages); u += step) {
-          const int t = u / p.splits, kb0 = (u % p.splits) * p.kb_per, kb1 = min(kblocks, kb0 + p.kb_per);
-          for (int kb = kb0; kb < kb1 && ahead < uint32_t(C::kStages); ++kb, ++ahead) {
-            mbar_arrive_expect_tx(&ring->full[ahead], C::kStageBytes);  // first use of every stage: it is empty
-            const uint32_t wdst = tiles_addr + ahead * C::kStageBytes + kABytes;
-            if (p.swiglu_i) {  // two boxes of 128 rows: gate rows, then up rows
-              tma_load_2d<kPair>(wdst, &map_w, kb * kBK, (t / mt) * tile_cols, smem_u32(&ring->full[ahead]));
-              tma_load_2d<kPair>(wdst + C::kWBytes / 2, &map_w, kb * kBK, p.swiglu_i + (t / mt) * tile_cols,
-                                 smem_u32(&ring->full[ahead]));
-            } else {
-              tma_load_2d<kPair>(wdst, &map_w, kb * kBK, (t / mt) * kBN, smem_u32(&ring->full[ahead]));
-            }
-          }
-        }
-        asm volatile("griddepcontrol.wait;" ::: "memory");
-      }
+      uint32_t s = 0, ph = 0;
       bool ok = true;
       for (int u = first; u < units && ok; u += step) {
         const int t = u / p.splits, kb0 = (u % p.splits) * p.kb_per, kb1 = min(kblocks, kb0 + p.kb_per);
         const int m0 = (t % mt) * C::kTileM + int(rank) * kBM;
-        // W rows of this CTA's block: its half (pair) or all (single) of the tile's 256 columns; with the
-        // fused SwiGLU, columns 0..127 are gate rows n0.. and columns 128..255 are up rows I + n0..
+        // W rows of this CTA's block: its half (pair) or all (single) of the tile's columns; with the fused
+        // SwiGLU, the first half of the columns are gate rows n0.. and the second half up rows I + n0..
         const int n0 = p.swiglu_i ? (t / mt) * tile_cols + (kPair && rank ? p.swiglu_i : 0)
-                                  : (t / mt) * kBN + int(rank) * C::kWRows;
-        for (int kb = kb0; kb < kb1; ++kb, ++it) {
-          const uint32_t s = it % C::kStages, ph = (it / C::kStages) & 1u;
-          const uint32_t dst = tiles_addr + s * C::kStageBytes, bar = full0 + s * uint32_t(sizeof(uint64_t));
-          if (it < ahead) {  // armed and half loaded above
+                                  : (t / mt) * bn + (kPair ? int(rank) * (bn / 2) : 0);
+        for (int kb = kb0; kb < kb1; ++kb, turn ^= 1u) {
+         if (turn == 0u) {
+          const uint32_t dst = tiles_addr + s * stage_bytes, bar = full0 + s * uint32_t(sizeof(uint64_t));
+          if (!(ok = wait_or_abort(&ring->empty[s], ph ^ 1u, ring, p.status))) break;
+          if (leader) mbar_arrive_expect_tx(&ring->full[s], (kPair ? 2u : 1u) * (is_a ? kABytes : w_bytes));
+          if (is_a) {
             tma_load_2d<kPair>(dst, &map_a, kb * kBK, m0, bar);
-            continue;
+          } else {
+            tma_load_2d<kPair>(dst + kABytes, &map_w, kb * kBK, n0, bar);
+            if (!kPair && p.swiglu_i)
+              tma_load_2d<kPair>(dst + kABytes + w_bytes / 2, &map_w, kb * kBK, p.swiglu_i + n0, bar);
           }
-          if (!(ok = wait_or_abort(&ring->empty[s], (kPair && !leader) ? ph : (ph ^ 1u), ring, p.status))) break;
-          if (leader) {
-            mbar_arrive_expect_tx(&ring->full[s], (kPair ? 2u : 1u) * C::kStageBytes);
-            if constexpr (kPair) mbar_arrive_remote(smem_u32(&ring->empty[s]), 1);
-          }
-          tma_load_2d<kPair>(dst, &map_a, kb * kBK, m0, bar);
-          tma_load_2d<kPair>(dst + kABytes, &map_w, kb * kBK, n0, bar);
-          if (!kPair && p.swiglu_i)
-            tma_load_2d<kPair>(dst + kABytes + C::kWBytes / 2, &map_w, kb * kBK, p.swiglu_i + n0, bar);
+         }
+          if (++s == stages) s = 0, ph ^= 1u;
         }
       }
     }
   } else if (warp == 1) {
-    if (lane == 0 && leader) {
-      uint32_t it = 0, local = 0;
+    if (leader) {  // the whole warp runs the loop, one lane issues
+      const uint32_t idesc = C::kIdescM | (uint32_t(bn >> 3) << 17);
+      uint32_t s = 0, ph = 0, local = 0;
       bool ok = true;
       for (int u = first; u < units && ok; u += step, ++local) {
         const int kb0 = (u % p.splits) * p.kb_per, kb1 = min(kblocks, kb0 + p.kb_per);
@@ -450,18 +599,24 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         if (!(ok = wait_or_abort(&ring->acc_empty[acc], aph ^ 1u, ring, p.status))) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * kBN;
-        for (int kb = kb0; kb < kb1; ++kb, ++it) {
-          const uint32_t s = it % C::kStages, ph = (it / C::kStages) & 1u;
+        for (int kb = kb0; kb < kb1; ++kb) {
           if (!(ok = wait_or_abort(&ring->full[s], ph, ring, p.status))) break;
           tc_fence_after();
-          const uint32_t a_addr = tiles_addr + s * C::kStageBytes;
+          const uint32_t a_addr = tiles_addr + s * stage_bytes;
           const uint64_t a_desc = smem_desc_k128(a_addr), w_desc = smem_desc_k128(a_addr + kABytes);
+          if (elect_one()) {
 #pragma unroll
-          for (int k = 0; k < kBK / 32; ++k)  // 32 bytes of K per instruction: +2 in 16-byte units
-            mma_f8<kPair>(d_tmem, a_desc + uint64_t(2 * k), w_desc + uint64_t(2 * k), C::kIdesc, (kb > kb0) || k != 0);
-          mma_commit<kPair>(smem_u32(&ring->empty[s]));
+            for (int k = 0; k < kBK / 32; ++k)  // 32 bytes of K per instruction: +2 in 16-byte units
+              mma_f8<kPair>(d_tmem, a_desc + uint64_t(2 * k), w_desc + uint64_t(2 * k), idesc, (kb > kb0) || k != 0);
+            if constexpr (kPair) mma_commit_both(smem_u32(&ring->empty[s])); else mma_commit<false>(smem_u32(&ring->empty[s]));
+          }
+          __syncwarp();
+          if (++s == stages) s = 0, ph ^= 1u;
         }
-        if (ok) mma_commit<kPair>(smem_u32(&ring->acc_full[acc]));
+        if (ok && elect_one()) {
+          if constexpr (kPair) mma_commit_both(smem_u32(&ring->acc_full[acc])); else mma_commit<false>(smem_u32(&ring->acc_full[acc]));
+        }
+        __syncwarp();
       }
     }
   } else {
@@ -470,27 +625,34 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     const int et = int(threadIdx.x) - 64;  // 0..127 among the epilogue threads
     uint32_t local = 0;
     bool ok = true;
+    const bool slabs = p.vec != 0 && p.splits == 1;  // the output can be moved by TMA
+    SlabState st{tiles_addr + C::kEpiOffset + uint32_t(warp - 2) * (2 * kSlabBytes), ring->res_full[warp - 2], 0u};
     for (int u = first; u < units && ok; u += step, ++local) {
       const int t = u / p.splits, sl = u % p.splits;
       const uint32_t acc = local & 1u, aph = (local >> 1) & 1u;
-      const int m0 = (t % mt) * C::kTileM + int(rank) * kBM, n0 = (t / mt) * tile_cols;
+      const int m0 = (t % mt) * C::kTileM + int(rank) * kBM, n0 = (t / mt) * tile_cols, row0 = m0 + q * 32;
+      const int n_end = min(p.swiglu_i ? p.swiglu_i : p.N, n0 + tile_cols);
+      const bool live = row0 < p.M;  // uniform over the warp: a warp whose rows are all past M has nothing to do
+      if (slabs && live && lane == 0 && p.out_kind == GRANITE4_GEMM_OUT_RESIDUAL) residual_ahead(&map_res, st, n0, n_end, row0);
       ok = wait_or_abort(&ring->acc_full[acc], aph, ring, p.status);
       if (p.splits > 1) ok = epilogue_all(ok);  // the split path below has barriers: leave it together or not at all
       if (!ok) break;
-      // the leader learns from its own barrier that both halves of the accumulator are complete
-      // and tells the peer
-      if (kPair && leader && warp == 2 && lane == 0) mbar_arrive_remote(smem_u32(&ring->acc_full[acc]), 1);
       tc_fence_after();
       float* partial = p.splits > 1 ? p.ws + (size_t(t) * p.splits + sl) * p.ws_rows * kBN : nullptr;
-      if (p.swiglu_i) {
-        if (m0 + q * 32 < p.M) {
-          const uint32_t amax = amax_warp(store_accumulator_swiglu(p, tmem_base + (uint32_t(q * 32) << 16) + acc * kBN,
-                                                                   m0 + q * 32 + lane, n0, a_scale));
+      const uint32_t taddr = tmem_base + (uint32_t(q * 32) << 16) + acc * kBN;
+      if (live) {
+        uint32_t amax = 0u;
+        if (slabs)
+          amax = store_slabs(p, &map_out, &map_res, st, ring, taddr, lane, row0, n0, n_end, bn / 2, a_scale, ok);
+        else if (p.swiglu_i)
+          amax = store_accumulator_swiglu(p, taddr, row0 + lane, n0, a_scale, bn / 2);
+        else
+          store_accumulator(p, taddr, row0 + lane, n0, bn, a_scale, partial != nullptr ? partial + size_t(q * 32 + lane) * kBN : nullptr);
+        if (p.swiglu_i) {
+          amax = amax_warp(amax);
           if (lane == 0 && amax != 0u) atomic_amax(p.amax_slot + 1, amax_value(amax));
         }
-      } else if (m0 + q * 32 < p.M)  // uniform over the warp: a warp whose rows are all past M has nothing to read
-        store_accumulator(p, tmem_base + (uint32_t(q * 32) << 16) + acc * kBN, m0 + q * 32 + lane, n0, a_scale,
-                          partial != nullptr ? partial + size_t(q * 32 + lane) * kBN : nullptr);
+      }
       tc_fence_before();
       __syncwarp();
       if (lane == 0) {
@@ -531,6 +693,8 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
       }
     }
   }
+
+  if (warp >= 2 && warp < 6 && lane == 0) bulk_wait_all<0>();  // this warp's stores have been performed
 
   // Wind down. On the normal path the epilogue has seen the last accumulator
   // complete, so no MMA and no copy is in flight. After an abort, give copies
@@ -593,7 +757,7 @@ gemm_fp8_stream_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t tiles_addr = (raw + 1023u) & ~1023u;
   StreamRing* ring = reinterpret_cast<StreamRing*>(smem_raw + (tiles_addr - raw) + kStreamTileBytes + (kBM - 16) * kBK);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const uint32_t a_blk = uint32_t(p.a_rows) * kBK, w_blk = uint32_t(p.bn) * kBK;
   const uint32_t stage_bytes = uint32_t(p.kc) * (a_blk + w_blk);
 
@@ -662,22 +826,20 @@ gemm_fp8_stream_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
       issue(it, true, true);
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      const uint32_t idesc = (1u << 4) | (uint32_t(p.bn >> 3) << 17) | (uint32_t(kBM >> 4) << 24);
-      long long it = 0;
-      uint32_t local = 0;
-      bool ok = true;
-      for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x, ++local) {
-        const uint32_t acc = local & 1u, aph = (local >> 1) & 1u;
-        if (!(ok = stream_wait(&ring->acc_empty[acc], aph ^ 1u, ring, p.status))) break;
+    const uint32_t idesc = (1u << 4) | (uint32_t(p.bn >> 3) << 17) | (uint32_t(kBM >> 4) << 24);
+    uint32_t s = 0, ph = 0, local = 0;
+    bool ok = true;
+    for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x, ++local) {
+      const uint32_t acc = local & 1u, aph = (local >> 1) & 1u;
+      if (!(ok = stream_wait(&ring->acc_empty[acc], aph ^ 1u, ring, p.status))) break;
+      tc_fence_after();
+      const uint32_t d_tmem = tmem_base + acc * kBN;
+      for (int st = 0; st < stages_per_tile; ++st) {
+        if (!(ok = stream_wait(&ring->full[s], ph, ring, p.status))) break;
         tc_fence_after();
-        const uint32_t d_tmem = tmem_base + acc * kBN;
-        for (int st = 0; st < stages_per_tile; ++st, ++it) {
-          const uint32_t s = uint32_t(it % p.stages), ph = uint32_t(it / p.stages) & 1u;
-          if (!(ok = stream_wait(&ring->full[s], ph, ring, p.status))) break;
-          tc_fence_after();
-          const uint32_t base = tiles_addr + s * stage_bytes;
-          const int nblk = min(p.kc, kblocks - st * p.kc);
+        const uint32_t base = tiles_addr + s * stage_bytes;
+        const int nblk = min(p.kc, kblocks - st * p.kc);
+        if (elect_one()) {
           for (int j = 0; j < nblk; ++j) {
             const uint64_t a_desc = smem_desc_k128(base + j * a_blk), w_desc = smem_desc_k128(base + p.kc * a_blk + j * w_blk);
 #pragma unroll
@@ -686,8 +848,11 @@ gemm_fp8_stream_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
           }
           mma_commit<false>(smem_u32(&ring->empty[s]));
         }
-        if (ok) mma_commit<false>(smem_u32(&ring->acc_full[acc]));
+        __syncwarp();
+        if (++s == uint32_t(p.stages)) s = 0, ph ^= 1u;
       }
+      if (ok && elect_one()) mma_commit<false>(smem_u32(&ring->acc_full[acc]));
+      __syncwarp();
     }
   } else {
     const int q = warp & 3;
@@ -743,45 +908,53 @@ gemm_fp8_stream_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
 // accumulator is 128 tensor-memory lanes (output columns) by 16 columns (output rows).
 //
 // A unit is 128 weight rows times a slice of K; the grid is one CTA per unit and is not persistent.
-// The CTA is small (a 90 KB ring, 32 columns of tensor memory) so that two are resident per SM: while
+// The CTA is small (a ring of 90 - 108 KB, 32 columns of tensor memory) so that two are resident per SM: while
 // one drains its accumulator the other streams, and under programmatic dependent launch the CTAs of
 // the next GEMM on the stream move in and fetch their first weight blocks while this one finishes.
 //
 // The slices of one tile are the CTAs of one thread-block cluster, and their partial sums meet in
 // distributed shared memory as a reduce-scatter: rank o owns a chunk of the tile's 128 columns; the
 // epilogue thread of every other rank that holds one of those columns stores its partial sums into
-// rank o's receive buffer and arrives (release, cluster scope) on rank o's mbarrier; the owner's
-// thread for the column waits for that barrier (acquire), adds the partials in rank order - its own
-// from registers in its place - and runs the epilogue. No workspace in global memory, no atomics,
+// rank o's receive buffer with st.async, whose bytes complete rank o's mbarrier (stores followed by a
+// release arrival per thread: 1.5 us from accumulator to sum, 0.9 now); the owner's thread for the column waits for that barrier
+// (acquire), adds the partials in rank order - its own from registers in its place - and runs the
+// epilogue. No workspace in global memory, no atomics,
 // the same order of additions every time, and no cluster-wide barrier on the way out: the only one
 // is at the start (every CTA is running and its barriers exist before anyone writes to it), where
 // it overlaps the first loads.
 //
-// Roles: warp 0, lanes 0 .. 4: lane s owns ring stage s (k-blocks s, s + 5, ...): arms its barrier and
-// issues the two TMA loads, the first W block before the wait on the kernel ahead of this one on the
-// stream; warp 1: tensor-memory allocation, one thread issues the MMAs; warps 2-5: accumulator ->
-// registers, exchange, epilogue. Every mbarrier wait is bounded as in the other forms.
-constexpr int kDecStages = 5, kDecRows = 16;
+// Roles: warps 0 and 6: W loaders (the first fill, then every second k-block each); warp 7: A loader, the only one that waits for
+// the kernel ahead on the stream; warp 1: tensor-memory allocation, one thread issues the MMAs; warps 2-5:
+// accumulator -> registers, exchange, epilogue. A thread gets through one tiled copy per ~0.27 us (ring
+// wait, expect_tx, issue) whatever its size - 61 B/ns for 16 KB boxes, measured with the data in L2 - and
+// the lanes of one warp take turns: with both operands of a stage issued from one warp a CTA was held to
+// 39 B/ns however far ahead the weights had been fetched. Three issuing warps and the MMA loop run by a
+// whole warp (elect_one): one row, gate|up 19.9 -> 17.4 us, down 12.6 -> 10.0, QKV 6.9 -> 5.7, O 6.2 -> 5.1.
+// Every mbarrier wait is bounded as in the other forms.
+constexpr int kDecMaxStages = 6, kDecRows = 16;
 constexpr uint32_t kDecWBytes = kBM * kBK, kDecABytes = kDecRows * kBK, kDecStageBytes = kDecWBytes + kDecABytes;
 constexpr uint32_t kDecTmemCols = 32;
 constexpr int kDecMaxSplits = 8;  // the portable cluster size
-constexpr uint32_t kDecRecvBytes = 10240;
-constexpr size_t kDecSmemBytes = 1024 + size_t(kDecStages) * kDecStageBytes + kDecRecvBytes + 256;
+// Dynamic shared memory of a CTA when two of them share an SM (228 KB, 1 KB of each taken by the system).
+constexpr size_t kDecSmemMax = 228 * 1024 / 2 - 1024;
 struct DecRing {
-  uint64_t full[kDecStages], empty[kDecStages], acc_full, red_full;
+  uint64_t full[kDecMaxStages], empty[kDecMaxStages], acc_full, red_full;
   uint32_t tmem_base;
   int abort;
 };
 
 // Columns of a tile owned by one rank of a cluster of `splits`: a multiple of 8, so that an owner's
-// bf16 row segment starts on a 16-byte boundary. (splits - 1) * 4 row groups * chunk * 16 bytes fit
-// in kDecRecvBytes for every splits <= 8.
+// bf16 row segment starts on a 16-byte boundary.
 __host__ __device__ constexpr int dec_chunk(int splits) { return ((kBM + splits - 1) / splits + 7) / 8 * 8; }
-static_assert(7 * 4 * dec_chunk(8) * 16 <= int(kDecRecvBytes) && 5 * 4 * dec_chunk(6) * 16 <= int(kDecRecvBytes) &&
-                  4 * 4 * dec_chunk(5) * 16 <= int(kDecRecvBytes) && 3 * 4 * dec_chunk(4) * 16 <= int(kDecRecvBytes) &&
-                  2 * 4 * dec_chunk(3) * 16 <= int(kDecRecvBytes) && 6 * 4 * dec_chunk(7) * 16 <= int(kDecRecvBytes) &&
-                  1 * 4 * dec_chunk(2) * 16 <= int(kDecRecvBytes),
-              "the receive buffer holds every rank's partial sums of the owned columns");
+// What the other ranks store for an owner: 16 bytes per sender, group of four rows and owned column.
+__host__ __device__ constexpr int dec_recv_bytes(int splits, int M) { return (splits - 1) * ((M + 3) / 4) * dec_chunk(splits) * 16; }
+constexpr size_t dec_smem_bytes(int stages, int splits, int M) {
+  return 1024 + size_t(stages) * kDecStageBytes + size_t(dec_recv_bytes(splits, M)) + 256;
+}
+// The ring takes what the receive buffer leaves: six stages up to eight rows, five above.
+constexpr int dec_stages(int splits, int M) { return dec_smem_bytes(kDecMaxStages, splits, M) <= kDecSmemMax ? kDecMaxStages : kDecMaxStages - 1; }
+static_assert(dec_smem_bytes(5, 8, 16) <= kDecSmemMax && dec_smem_bytes(5, 6, 16) <= kDecSmemMax && dec_smem_bytes(6, 6, 8) <= kDecSmemMax,
+              "two CTAs of the 16-row form share an SM");
 
 __device__ __forceinline__ bool dec_wait(uint64_t* bar, uint32_t parity, DecRing* ring, unsigned int* status) {
   volatile int* ab = &ring->abort;
@@ -827,16 +1000,18 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
       : "memory");
 }
 
-__global__ void __launch_bounds__(kThreads, 2)
+constexpr int kDecThreads = 256;
+__global__ void __launch_bounds__(kDecThreads, 2)
 gemm_fp8_decode_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
                        const GemmParams p) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t tiles_addr = (raw + 1023u) & ~1023u;
   uint8_t* tiles_ptr = smem_raw + (tiles_addr - raw);
-  uint8_t* recv_ptr = tiles_ptr + size_t(kDecStages) * kDecStageBytes;
-  DecRing* ring = reinterpret_cast<DecRing*>(recv_ptr + kDecRecvBytes);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int stages = p.stages;
+  uint8_t* recv_ptr = tiles_ptr + size_t(stages) * kDecStageBytes;
+  DecRing* ring = reinterpret_cast<DecRing*>(recv_ptr + dec_recv_bytes(p.splits, p.M));
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int splits = p.splits;
   const uint32_t rank = splits > 1 ? cluster_rank() : 0u;  // the slice of K
   const int tile = int(blockIdx.x) / splits;
@@ -848,11 +1023,13 @@ gemm_fp8_decode_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
   if (threadIdx.x == 0) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&map_w)) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&map_a)) : "memory");
-    for (int s = 0; s < kDecStages; ++s) mbar_init(&ring->full[s], 1), mbar_init(&ring->empty[s], 1);
+    for (int s = 0; s < stages; ++s) mbar_init(&ring->full[s], 2), mbar_init(&ring->empty[s], 1);  // W loader, A loader
     mbar_init(&ring->acc_full, 1);
-    mbar_init(&ring->red_full, uint32_t(max(1, (splits - 1) * owned)));  // one arrival per partial column
+    mbar_init(&ring->red_full, 1);
     ring->abort = 0;
     mbar_init_fence();
+    // completed by the bytes the other ranks store for the owned columns (a rank that owns none gets none)
+    mbar_arrive_expect_tx(&ring->red_full, uint32_t((splits - 1) * ((p.M + 3) / 4) * owned * 16));
     fence_async_smem();
   }
   if (warp == 1) tmem_alloc<false>(smem_u32(&ring->tmem_base), kDecTmemCols);
@@ -868,46 +1045,50 @@ gemm_fp8_decode_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
   // what the kernel ahead wrote (activations, their scale, the residual) or that write wait for it.
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
-  if (warp == 0) {
-    if (lane < kDecStages) {
-      const uint32_t dst = tiles_addr + uint32_t(lane) * kDecStageBytes, bar = smem_u32(&ring->full[lane]);
-      int kb = kb0 + lane;
-      const bool any = kb < kb1;
-      if (any) {  // first use of the stage: it is empty; W is a constant of the model
-        mbar_arrive_expect_tx(&ring->full[lane], kDecStageBytes);
-        tma_load_2d<false>(dst, &map_w, kb * kBK, tile * kBM, bar);
-      }
-      asm volatile("griddepcontrol.wait;" ::: "memory");
-      if (any) tma_load_2d<false>(dst + kDecWBytes, &map_a, kb * kBK, 0, bar);
-      uint32_t round = 1;
-      for (kb += kDecStages; kb < kb1; kb += kDecStages, ++round) {
-        if (!dec_wait(&ring->empty[lane], (round & 1u) ^ 1u, ring, p.status)) break;
-        mbar_arrive_expect_tx(&ring->full[lane], kDecStageBytes);
-        tma_load_2d<false>(dst, &map_w, kb * kBK, tile * kBM, bar);
-        tma_load_2d<false>(dst + kDecWBytes, &map_a, kb * kBK, 0, bar);
+  if (warp == 0 || warp >= 6) {
+    const bool is_a = warp == 7;
+    const CUtensorMap* map = is_a ? &map_a : &map_w;
+    const uint32_t bytes = is_a ? kDecABytes : kDecWBytes, at = is_a ? kDecWBytes : 0u;
+    const int row = is_a ? 0 : tile * kBM;
+    auto load = [&](int i, uint32_t s) {  // k-block kb0 + i into stage s
+      mbar_arrive_expect_tx(&ring->full[s], bytes);
+      tma_load_2d<false>(tiles_addr + s * kDecStageBytes + at, map, (kb0 + i) * kBK, row, smem_u32(&ring->full[s]));
+    };
+    if (is_a) asm volatile("griddepcontrol.wait;" ::: "memory");  // W is a constant of the model
+    if (warp != 6 && lane < stages && kb0 + lane < kb1) load(lane, uint32_t(lane));  // the first fill: every stage is empty
+    __syncwarp();
+    if (lane == 0) {
+      const int step = is_a ? 1 : 2;
+      int i = stages + (warp == 6 ? 1 : 0);
+      uint32_t s = warp == 6 ? 1u : 0u, ph = 0u;
+      for (; kb0 + i < kb1; i += step) {
+        if (!dec_wait(&ring->empty[s], ph, ring, p.status)) break;
+        load(i, s);
+        if ((s += uint32_t(step)) >= uint32_t(stages)) s -= uint32_t(stages), ph ^= 1u;
       }
     }
     __syncwarp();
     if (splits > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
   } else if (warp == 1) {
-    if (lane == 0) {
-      // f32 accumulator, e4m3 x e4m3, both operands K-major, N 16, M 128
-      constexpr uint32_t idesc = (1u << 4) | (uint32_t(kDecRows >> 3) << 17) | (uint32_t(kBM >> 4) << 24);
-      uint32_t it = 0;
-      bool ok = true;
-      for (int kb = kb0; kb < kb1 && ok; ++kb, ++it) {
-        const uint32_t s = it % kDecStages, ph = (it / kDecStages) & 1u;
-        if (!(ok = dec_wait(&ring->full[s], ph, ring, p.status))) break;
-        tc_fence_after();
-        const uint32_t w_addr = tiles_addr + s * kDecStageBytes;
-        const uint64_t w_desc = smem_desc_k128(w_addr), a_desc = smem_desc_k128(w_addr + kDecWBytes);
+    // f32 accumulator, e4m3 x e4m3, both operands K-major, N 16, M 128; the whole warp runs the loop
+    constexpr uint32_t idesc = (1u << 4) | (uint32_t(kDecRows >> 3) << 17) | (uint32_t(kBM >> 4) << 24);
+    uint32_t it = 0, s = 0, ph = 0;
+    bool ok = true;
+    for (int kb = kb0; kb < kb1 && ok; ++kb, ++it) {
+      if (!(ok = dec_wait(&ring->full[s], ph, ring, p.status))) break;
+      tc_fence_after();
+      const uint32_t w_addr = tiles_addr + s * kDecStageBytes;
+      const uint64_t w_desc = smem_desc_k128(w_addr), a_desc = smem_desc_k128(w_addr + kDecWBytes);
+      if (elect_one()) {
 #pragma unroll
         for (int k = 0; k < kBK / 32; ++k)
           mma_f8<false>(tmem_base, w_desc + uint64_t(2 * k), a_desc + uint64_t(2 * k), idesc, (it | uint32_t(k)) != 0u);
         mma_commit<false>(smem_u32(&ring->empty[s]));
       }
-      if (ok) mma_commit<false>(smem_u32(&ring->acc_full));
+      __syncwarp();
+      if (++s == uint32_t(stages)) s = 0, ph ^= 1u;
     }
+    if (ok && elect_one()) mma_commit<false>(smem_u32(&ring->acc_full));
     __syncwarp();
     if (splits > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
   } else {
@@ -942,21 +1123,20 @@ gemm_fp8_decode_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
         // slot of this rank among the owner's senders: ranks in order, the owner itself left out
         const uint32_t slot = rank < uint32_t(owner) ? rank : rank - 1u;
         const uint32_t base = cluster_addr(smem_u32(recv_ptr), uint32_t(owner));
+        const uint32_t red = cluster_addr(smem_u32(&ring->red_full), uint32_t(owner));
 #pragma unroll
         for (int g = 0; g < kDecRows / 4; ++g) {
           if (g < groups) {
-            const uint32_t dst = base + (((slot * (kDecRows / 4) + uint32_t(g)) * uint32_t(chunk) + uint32_t(local)) << 4);
-            asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst), "r"(v[4 * g]),
-                         "r"(v[4 * g + 1]), "r"(v[4 * g + 2]), "r"(v[4 * g + 3])
-                         : "memory");
+            const uint32_t dst = base + (((slot * uint32_t(groups) + uint32_t(g)) * uint32_t(chunk) + uint32_t(local)) << 4);
+            asm volatile(
+                "st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(dst),
+                "r"(v[4 * g]), "r"(v[4 * g + 1]), "r"(v[4 * g + 2]), "r"(v[4 * g + 3]), "r"(red)
+                : "memory");
           }
         }
-        asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(
-                         cluster_addr(smem_u32(&ring->red_full), uint32_t(owner)))
-                     : "memory");
       } else {
         ok = ok && dec_wait_cluster(&ring->red_full, 0u, ring, p.status);
-        const float4* red = reinterpret_cast<const float4*>(recv_ptr);
+        const float4* got = reinterpret_cast<const float4*>(recv_ptr);
         float acc[kDecRows];
 #pragma unroll
         for (int j = 0; j < kDecRows; ++j) acc[j] = 0.0f;
@@ -971,7 +1151,7 @@ gemm_fp8_decode_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
                 x = make_float4(__uint_as_float(v[4 * g]), __uint_as_float(v[4 * g + 1]), __uint_as_float(v[4 * g + 2]),
                                 __uint_as_float(v[4 * g + 3]));
               else
-                x = red[(size_t(slot) * (kDecRows / 4) + g) * chunk + local];
+                x = got[(size_t(slot) * groups + g) * chunk + local];
               if (first) {
                 acc[4 * g] = x.x, acc[4 * g + 1] = x.y, acc[4 * g + 2] = x.z, acc[4 * g + 3] = x.w;
               } else {
@@ -1051,6 +1231,19 @@ bool make_map(CUtensorMap* map, const void* base, int rows, int K, long long ld,
 }
 
 
+// The output (or residual) matrix, moved in slabs of 32 rows x 128 bytes.
+bool make_slab_map(CUtensorMap* map, const void* base, int rows, int cols, long long ld, bool f32) {
+  EncodeTiledFn enc = encode_tiled();
+  if (enc == nullptr) return false;
+  const cuuint64_t dims[2] = {cuuint64_t(cols), cuuint64_t(rows)};
+  const cuuint64_t strides[1] = {cuuint64_t(ld) * (f32 ? 4 : 2)};
+  const cuuint32_t box[2] = {f32 ? 32u : 64u, 32u};
+  const cuuint32_t elem[2] = {1, 1};
+  return enc(map, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims,
+             strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 bool box3d_enabled() {
   const char* v = std::getenv("G4_GEMM_BOX3D");
   return !(v != nullptr && v[0] == '0');
@@ -1086,7 +1279,7 @@ cudaError_t smem_opt_in() {
 cudaLaunchConfig_t pair_config(int clusters) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(2u * unsigned(clusters));
-  cfg.blockDim = dim3(kThreads);
+  cfg.blockDim = dim3(kTileThreads);
   cfg.dynamicSmemBytes = CfgPair::kSmemBytes;
   return cfg;
 }
@@ -1114,6 +1307,29 @@ int pair_clusters() {
   (void)cudaGetLastError();
   known[dev] = fit;
   return fit;
+}
+
+// Columns of a pair tile: the width whose rounds of tiles over the CTA pairs take the least time. A k-block
+// takes the longer of its MMAs (0.30 us at 256 columns, clock 1.9 GHz) and what issuing, fetching and
+// handing over a stage costs; measured per k-block on a 12800-deep projection of 256 rows: 0.16 us at 64
+// columns, 0.19 at 128, 0.265 at 192, 0.33 at 256. The last round's epilogue and the start add the same
+// ~5 us to every choice. Widths are whole slabs of the epilogue (64 bf16 columns; the fused SwiGLU has
+// half as many output columns). Wider wins a tie: fewer A blocks. 500 rows, QKV: 256 columns 17.3 us (48
+// tiles on 74 pairs), 192: 14.7 (64 tiles), 128: 16.7 (two rounds); O: 256: 17.6, 128: 11.6 us.
+int plan_pair_columns(const GemmParams& p, int pairs) {
+  static constexpr int kWidth[4] = {256, 192, 128, 64};
+  static constexpr double kUs[4] = {0.33, 0.265, 0.19, 0.16};
+  const int mt = (p.M + 2 * kBM - 1) / (2 * kBM);
+  int best = kBN;
+  double least = 1e300;
+  for (int i = 0; i < 4; ++i) {
+    if (p.swiglu_i && kWidth[i] % 128 != 0) continue;
+    const int cols = p.swiglu_i ? kWidth[i] / 2 : kWidth[i], n = p.swiglu_i ? p.swiglu_i : p.N;
+    const long long tiles = 1ll * mt * ((n + cols - 1) / cols);
+    const double us = double((tiles + pairs - 1) / pairs) * p.kb_per * kUs[i];
+    if (us < least * 0.999) least = us, best = kWidth[i];
+  }
+  return best;
 }
 
 // Split of K for at most 16 rows of A. With T = ceil(N / 256) tiles and S slices of K there are
@@ -1242,7 +1458,7 @@ DecodePlan plan_decode(int N, int K, int sms) {
 // caller then takes another form), 0 launched, -1 failed.
 int launch_decode(const char* fn, const uint8_t* d_a, long long lda, const uint8_t* d_w, GemmParams p) {
   const DecodePlan pl = plan_decode(p.N, p.K, sm_count());
-  p.splits = pl.splits, p.kb_per = pl.kb_per;
+  p.splits = pl.splits, p.kb_per = pl.kb_per, p.stages = dec_stages(pl.splits, p.M);
   static std::mutex mu;
   static std::map<int, cudaError_t> done;
   static std::map<std::pair<int, int>, bool> fits;
@@ -1251,8 +1467,8 @@ int launch_decode(const char* fn, const uint8_t* d_a, long long lda, const uint8
   const int tiles = (p.N + kBM - 1) / kBM;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(unsigned(tiles) * unsigned(p.splits));
-  cfg.blockDim = dim3(kThreads);
-  cfg.dynamicSmemBytes = kDecSmemBytes;
+  cfg.blockDim = dim3(kDecThreads);
+  cfg.dynamicSmemBytes = dec_smem_bytes(p.stages, p.splits, p.M);
   cfg.stream = current_stream();
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -1264,7 +1480,7 @@ int launch_decode(const char* fn, const uint8_t* d_a, long long lda, const uint8
     std::lock_guard<std::mutex> lock(mu);
     if (done.find(dev) == done.end())
       done[dev] = cudaFuncSetAttribute(gemm_fp8_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       int(kDecSmemBytes));
+                                       int(kDecSmemMax));
     G4_CUDA_TRY(fn, done[dev]);
     const auto key = std::make_pair(dev, p.splits);
     if (fits.find(key) == fits.end()) {
@@ -1285,15 +1501,23 @@ int launch_decode(const char* fn, const uint8_t* d_a, long long lda, const uint8
 
 // Encodes the two tensor maps of form C and launches it over min(units, SMs) CTAs (CTA pairs).
 template <class C>
-int launch(const char* fn, const uint8_t* d_a, long long lda, const uint8_t* d_w, const GemmParams& p) {
+int launch(const char* fn, const uint8_t* d_a, long long lda, const uint8_t* d_w, GemmParams p) {
   constexpr bool kPair = C::kTileM == 2 * kBM;
-  CUtensorMap map_a, map_w;
+  if (!kPair) p.bn = kBN;
+  CUtensorMap map_a, map_w, map_out{}, map_res{};
   // the fused SwiGLU fetches a single CTA's 256 W rows as two boxes of 128 (gate rows, up rows)
-  const int w_box = (p.swiglu_i && !kPair) ? kBN / 2 : C::kWRows;
+  const int w_box = kPair ? p.bn / 2 : (p.swiglu_i ? kBN / 2 : kBN);
   if (!make_map(&map_a, d_a, p.M, p.K, lda, C::kARows) || !make_map(&map_w, d_w, p.N, p.K, p.K, w_box))
     return fail(fn, "the tensor map could not be encoded");
+  if (p.vec) {
+    const bool f32 = p.out_kind == GRANITE4_GEMM_OUT_F32;
+    const int cols = p.swiglu_i ? p.swiglu_i : p.N;
+    if (!make_slab_map(&map_out, f32 ? static_cast<const void*>(p.out_f32) : p.out_bf16, p.M, cols, p.ldc, f32) ||
+        (p.out_kind == GRANITE4_GEMM_OUT_RESIDUAL && !make_slab_map(&map_res, p.residual, p.M, cols, p.ldc, false)))
+      return fail(fn, "the tensor map could not be encoded");
+  }
   G4_CUDA_TRY(fn, smem_opt_in<C>());
-  const int nt = p.swiglu_i ? (p.swiglu_i + kBN / 2 - 1) / (kBN / 2) : (p.N + kBN - 1) / kBN;
+  const int tile_cols = p.swiglu_i ? p.bn / 2 : p.bn, nt = ((p.swiglu_i ? p.swiglu_i : p.N) + tile_cols - 1) / tile_cols;
   const int units = ((p.M + C::kTileM - 1) / C::kTileM) * nt * p.splits;
   if constexpr (kPair) {
     const int clusters = units < pair_clusters() ? units : pair_clusters();
@@ -1306,10 +1530,11 @@ int launch(const char* fn, const uint8_t* d_a, long long lda, const uint8_t* d_w
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = pdl_enabled() ? 2u : 1u;
-    G4_CUDA_TRY(fn, cudaLaunchKernelEx(&cfg, gemm_fp8_kernel<C>, map_a, map_w, p));
+    G4_CUDA_TRY(fn, cudaLaunchKernelEx(&cfg, gemm_fp8_kernel<C>, map_a, map_w, map_out, map_res, p));
   } else {
     const int grid = units < sm_count() ? units : sm_count();
-    G4_LAUNCH_PDL(fn, gemm_fp8_kernel<C>, dim3(grid), dim3(kThreads), C::kSmemBytes, current_stream(), map_a, map_w, p);
+    G4_LAUNCH_PDL(fn, gemm_fp8_kernel<C>, dim3(grid), dim3(kTileThreads), C::kSmemBytes, current_stream(), map_a, map_w,
+                  map_out, map_res, p);
   }
   return 0;
 }
@@ -1389,6 +1614,9 @@ extern "C" int granite4_kernel_gemm_fp8(int out_kind, const uint8_t* d_a, long l
   }
   // 256-row tiles on CTA pairs where the device co-schedules two-CTA clusters of this size
   // (G4_GEMM_PAIR=0 keeps the single form)
-  if (pair_enabled() && pair_clusters() > 0) return launch<CfgPair>(fn, d_a, lda, d_w, p);
+  if (pair_enabled() && pair_clusters() > 0) {
+    p.bn = plan_pair_columns(p, pair_clusters());
+    return launch<CfgPair>(fn, d_a, lda, d_w, p);
+  }
   return launch<CfgWide>(fn, d_a, lda, d_w, p);
 }

@@ -42,3 +42,71 @@ def test_fp8_codes_of_every_bf16_value_under_every_amax_mantissa(K, port, expone
         assert sa[1].item() == amax and sa[0].item() == scale
         got = codes.cpu().numpy()
         assert (got == want).all(), (m, (got != want).sum())
+
+
+def _exact_gemm_case(K, M, N, Kd, kind, pad=0):
+    """Codes from {0, +-1, +-2} make every sum exact in f32, so every form of the GEMM must return the
+    integer result exactly (bf16: rounded once), whatever order it adds in."""
+    g = torch.Generator(device=DEV).manual_seed(M * 7919 + N * 31 + Kd)
+    vals = torch.tensor([0x00, 0x38, 0xB8, 0x40, 0xC0], dtype=torch.uint8, device=DEV)  # 0, 1, -1, 2, -2
+
+    def codes(r, c):
+        return vals[torch.randint(5, (r, c), generator=g, device=DEV)]
+    a, w = codes(M, Kd), codes(N, Kd)
+    num = {0x00: 0.0, 0x38: 1.0, 0xB8: -1.0, 0x40: 2.0, 0xC0: -2.0}
+    lut = torch.zeros(256, device=DEV)
+    for c, v in num.items():
+        lut[c] = v
+    want = (lut[a.long()].double() @ lut[w.long()].double().T)
+    ldc = (N + 7) // 8 * 8 + pad
+    buf = torch.full((M, ldc), 7.0, dtype=torch.float32 if kind == "f32" else torch.bfloat16, device=DEV)
+    out = buf[:, :N]
+    res = None
+    if kind == "residual":
+        rbuf = torch.randint(-8, 8, (M, ldc), generator=g, device=DEV).to(torch.bfloat16)
+        res = rbuf[:, :N]
+        want = want * 0.5 + res.double()
+    ws = K.gemm_fp8_workspace(M, N, Kd, DEV)
+    assert K.gemm_fp8(a, w, out, residual=res, resid_scale=0.5, workspace=ws) == 0
+    want = want.float() if kind == "f32" else want.float().to(torch.bfloat16)
+    assert torch.equal(out, want), (M, N, Kd, kind)
+    assert (buf[:, N:] == 7.0).all()  # nothing past column N
+
+
+# row counts at the edges of the forms and of their 128- / 256-row tiles; widths that plan 64, 128, 192 and
+# 256 columns, with ragged last slabs; K of one block, of more blocks than the ring, not a multiple of 128
+@pytest.mark.parametrize("M", [1, 8, 9, 16, 17, 33, 128, 129, 255, 256, 257, 500])
+@pytest.mark.parametrize("N,Kd", [(72, 128), (1000, 1552), (4096, 512), (6144, 256)])
+def test_gemm_forms_are_exact_at_their_edges(K, M, N, Kd):
+    for kind in ("bf16", "f32", "residual"):
+        _exact_gemm_case(K, M, N, Kd, kind, pad=8 if kind == "residual" else 0)
+
+
+@pytest.mark.parametrize("rows", [1, 2, 3, 5, 8, 9, 15, 16, 17])
+@pytest.mark.parametrize("cols", [8, 264, 4096, 8184, 8192])
+def test_small_norm_quant_and_swiglu_equal_the_oracle(K, port, rows, cols):
+    """The one-launch forms of a decode step (one CTA, or one cluster) and the first row count past them."""
+    rng = np.random.default_rng(rows * 10007 + cols)
+
+    def bf(shape, sigma=1.0):
+        return ((sigma * rng.standard_normal(shape)).astype(np.float32).view(np.uint32) >> 16).astype(np.uint16)
+    y, res, w = bf((rows, cols)), bf((rows, cols)), bf(cols, 0.1) + 0  # weights of either sign
+    h, n = port.add_rmsnorm(y, res, w, 1e-5, 0.22)
+    codes, scale, amax = port.quant_fp8(n)
+    ho, no = (torch.empty(rows, cols, dtype=torch.int16, device=DEV) for _ in range(2))
+    c8 = torch.empty(rows, cols, dtype=torch.uint8, device=DEV)
+    sa, rstd = torch.full((2,), 9.0, device=DEV), torch.empty(rows, device=DEV)
+    assert K.add_rmsnorm_fp8(dev(y), dev(res), dev(w), 1e-5, 0.22, ho, no, c8, sa, rstd) == 0
+    assert (ho.cpu().numpy().view(np.uint16) == h).all() and (no.cpu().numpy().view(np.uint16) == n).all()
+    assert (c8.cpu().numpy() == codes).all() and sa[0].item() == scale and sa[1].item() == amax
+    cq, sw, aw = port.quant_fp8(y)
+    assert K.fp8_quant(dev(y), c8, sa) == 0
+    assert (c8.cpu().numpy() == cq).all() and sa[0].item() == sw and sa[1].item() == aw
+    act = torch.empty(rows, cols, dtype=torch.int16, device=DEV)
+    assert K.swiglu_fp8(dev(y), dev(res), act, c8, sa) == 0
+    got = act.cpu().numpy().view(np.uint16)
+    want = port.swiglu((y.astype(np.uint32) << 16).view(np.float32), (res.astype(np.uint32) << 16).view(np.float32))
+    key = lambda x: np.where(x & 0x8000, -(x.astype(np.int32) & 0x7FFF), x.astype(np.int32))  # noqa: E731
+    assert np.abs(key(got) - key(want)).max() <= 1  # the stated 1 bf16 ulp
+    cs, ss, as_ = port.quant_fp8(got)
+    assert (c8.cpu().numpy() == cs).all() and sa[0].item() == ss and sa[1].item() == as_
