@@ -74,7 +74,6 @@ constexpr int kRaw = 3;   // raw stages
 
 constexpr uint32_t kQTileBytes = 128 * kD * 2;     // 32768: two 64-dim halves of [128 rows][128 bytes]
 constexpr uint32_t kKvTileBytes = kTN * kD * 2;    // 16384: two 64-dim halves of [64 positions][128 bytes]
-constexpr uint32_t kPTileBytes = 128 * kTN * 2;    // 16384: [128 rows][128 bytes]
 constexpr uint32_t kRawBytes = kTN * kD;           // 8192 per matrix and stage
 
 struct TcSmem {
@@ -128,36 +127,6 @@ __device__ __forceinline__ void mma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uin
       "setp.ne.b32 p, %4, 0;\n\t"
       "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem),
       "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// Four MMAs of one accumulator in one statement: D (+)= A0 B0 + A1 B1 + A2 B2 + A3 B3; `accumulate` = 0
-// makes the first of them overwrite D.
-__device__ __forceinline__ void mma4_ss(uint32_t d_tmem, uint64_t a0, uint64_t b0, uint64_t a1, uint64_t b1, uint64_t a2,
-                                        uint64_t b2, uint64_t a3, uint64_t b3, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\t"
-      "setp.ne.b32 p, %10, 0;\n\t"
-      "setp.eq.b32 q, 0, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %9, p;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %3, %4, %9, q;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %5, %6, %9, q;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %7, %8, %9, q;\n\t}" ::"r"(d_tmem),
-      "l"(a0), "l"(b0), "l"(a1), "l"(b1), "l"(a2), "l"(b2), "l"(a3), "l"(b3), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// The same with A in tensor memory: k-step i reads the 8 columns from a_tmem + 8 i.
-__device__ __forceinline__ void mma4_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b0, uint64_t b1, uint64_t b2, uint64_t b3,
-                                        uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\t.reg .b32 a1, a2, a3;\n\t"
-      "setp.ne.b32 p, %7, 0;\n\t"
-      "setp.eq.b32 q, 0, 0;\n\t"
-      "add.u32 a1, %1, 8;\n\tadd.u32 a2, %1, 16;\n\tadd.u32 a3, %1, 24;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %6, p;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [a1], %3, %6, q;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [a2], %4, %6, q;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [a3], %5, %6, q;\n\t}" ::"r"(d_tmem),
-      "r"(a_tmem), "l"(b0), "l"(b1), "l"(b2), "l"(b3), "r"(idesc), "r"(accumulate)
       : "memory");
 }
 // A shared-memory descriptor from its two words (g4_tcgen05.cuh smem_desc_sw128): the low one holds the
@@ -230,7 +199,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_prefill_tc_kernel(const TcPa
   pdl_begin();
   extern __shared__ uint8_t smem_raw[];
   TcSmem* sm = reinterpret_cast<TcSmem*>(smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u));
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int hkv = blockIdx.y;
   // the longest prefixes first
   const int blk = static_cast<int>(gridDim.x) - 1 - static_cast<int>(blockIdx.x);
@@ -321,51 +290,46 @@ __global__ void __launch_bounds__(kThreads, 1) attn_prefill_tc_kernel(const TcPa
     }
   } else if (warp == 1) {
     // ---- MMA issue ----------------------------------------------------------------------------
-    // One thread issues every MMA; it is the busiest thread of the CTA (29 MMAs and commits per
-    // tile), so its instruction count per MMA is kept at the minimum: the descriptors of Q are
-    // formed once, those of a tile's K and V once per tile (both row tiles use them), and four MMAs
-    // go out per asm statement.
-    if (lane == 0) {
-      bool ok = wait_tc(&sm->q_ready, 0, sm, p.status);
-      const uint32_t q_lo = (smem_u32(sm->q16[0]) >> 4) | (1u << 16), k_lo = (smem_u32(sm->k16[0]) >> 4) | (1u << 16);
-      const uint32_t v_lo = (smem_u32(sm->v16[0]) >> 4) | ((kKvTileBytes / 2 >> 4) << 16);  // 64-dim halves 8 KB apart
-      uint64_t qd[kRowTiles][8];
-#pragma unroll
-      for (int t = 0; t < kRowTiles; ++t)
-#pragma unroll
-        for (int kk = 0; kk < 8; ++kk)  // 16 dims = 32 bytes per instruction; dims 64.. in the second half tile
-          qd[t][kk] = desc_of(q_lo + ((t * kQTileBytes + (kk >> 2) * (kQTileBytes / 2) + (kk & 3) * 32) >> 4));
-      auto issue_s = [&](int j) {
-        const int b = j % kBufs, sb = j & 1;
-        if (!(ok = ok && wait_tc(&sm->kv_full[b], (j / kBufs) & 1, sm, p.status))) return;
-        tc_fence_after();
-        uint64_t kd[8];
-#pragma unroll
-        for (int kk = 0; kk < 8; ++kk)
-          kd[kk] = desc_of(k_lo + ((b * kKvTileBytes + (kk >> 2) * (kKvTileBytes / 2) + (kk & 3) * 32) >> 4));
+    // The warp runs the loop together and one lane issues every MMA (elect_one): the descriptors stay in
+    // uniform registers. With the loop under `if (lane == 0)` an MMA held the thread for ~45 ns, 24 of them
+    // most of a tile's 1.85 us: a prefill chunk of 1999 rows after 30000 positions took 1675 us, 1400 now, 8192 rows from 0 906 and 760.
+    bool ok = wait_tc(&sm->q_ready, 0, sm, p.status);
+    const uint32_t q_lo = (smem_u32(sm->q16[0]) >> 4) | (1u << 16), k_lo = (smem_u32(sm->k16[0]) >> 4) | (1u << 16);
+    const uint32_t v_lo = (smem_u32(sm->v16[0]) >> 4) | ((kKvTileBytes / 2 >> 4) << 16);  // 64-dim halves 8 KB apart
+    auto issue_s = [&](int j) {
+      const int b = j % kBufs, sb = j & 1;
+      if (!(ok = ok && wait_tc(&sm->kv_full[b], (j / kBufs) & 1, sm, p.status))) return;
+      tc_fence_after();
+      if (elect_one()) {
 #pragma unroll
         for (int t = 0; t < kRowTiles; ++t) {
-          mma4_ss(tmem_base + s_col(t, sb), qd[t][0], kd[0], qd[t][1], kd[1], qd[t][2], kd[2], qd[t][3], kd[3], kIdescS, 0u);
-          mma4_ss(tmem_base + s_col(t, sb), qd[t][4], kd[4], qd[t][5], kd[5], qd[t][6], kd[6], qd[t][7], kd[7], kIdescS, 1u);
+#pragma unroll
+          for (int kk = 0; kk < 8; ++kk)  // 16 dims = 32 bytes per instruction; dims 64.. in the second half tile
+            mma_f16_ss(tmem_base + s_col(t, sb), desc_of(q_lo + ((t * kQTileBytes + (kk >> 2) * (kQTileBytes / 2) + (kk & 3) * 32) >> 4)),
+                       desc_of(k_lo + ((b * kKvTileBytes + (kk >> 2) * (kKvTileBytes / 2) + (kk & 3) * 32) >> 4)), kIdescS, kk > 0 ? 1u : 0u);
           mma_commit<false>(smem_u32(&sm->s_full[t][sb]));
         }
-      };
-      if (ok) issue_s(0);
-      for (int j = 0; j < n_kv && ok; ++j) {
-        if (j + 1 < n_kv) issue_s(j + 1);
-        const int b = j % kBufs, sb = j & 1;
-        uint64_t vd[4];
+      }
+      __syncwarp();
+    };
+    if (ok) issue_s(0);
+    for (int j = 0; j < n_kv && ok; ++j) {
+      if (j + 1 < n_kv) issue_s(j + 1);
+      const int b = j % kBufs, sb = j & 1;
+      for (int t = 0; t < kRowTiles && ok; ++t) {
+        if (!(ok = wait_tc(&sm->p_full[t][sb], (j >> 1) & 1, sm, p.status))) break;
+        tc_fence_after();
+        if (elect_one()) {
 #pragma unroll
-        for (int kk = 0; kk < 4; ++kk)  // 16 positions per instruction: 8 columns of P, two 8-row groups of V
-          vd[kk] = desc_of(v_lo + ((b * kKvTileBytes + kk * 2048) >> 4));
-        for (int t = 0; t < kRowTiles && ok; ++t) {
-          if (!(ok = wait_tc(&sm->p_full[t][sb], (j >> 1) & 1, sm, p.status))) break;
-          tc_fence_after();
-          mma4_ts(tmem_base + o_col(t), tmem_base + s_col(t, sb), vd[0], vd[1], vd[2], vd[3], kIdescPV, j > 0 ? 1u : 0u);
+          for (int kk = 0; kk < 4; ++kk)  // 16 positions per instruction: 8 columns of P, two 8-row groups of V
+            mma_f16_ts(tmem_base + o_col(t), tmem_base + s_col(t, sb) + kk * 8, desc_of(v_lo + ((b * kKvTileBytes + kk * 2048) >> 4)),
+                       kIdescPV, (j > 0 || kk > 0) ? 1u : 0u);
           mma_commit<false>(smem_u32(&sm->pv_done[t][sb]));
         }
-        if (ok) mma_commit<false>(smem_u32(&sm->kv_empty[b]));
+        __syncwarp();
       }
+      if (ok && elect_one()) mma_commit<false>(smem_u32(&sm->kv_empty[b]));
+      __syncwarp();
     }
   } else if (warp < 4 || warp >= 12) {
     // ---- converters -----------------------------------------------------------------------------
