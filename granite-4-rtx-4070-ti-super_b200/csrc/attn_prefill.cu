@@ -493,13 +493,13 @@ int attn_prefill_tc(const char* fn, const uint16_t* d_q, float scale, int Hq, in
                     const float* d_vs, const int* d_pt);
 
 // Launch of the flash form for a whole chunk; arguments as granite4_prefill_attention_int8 (validated there).
-// Chunks of 64 rows or more run on the tcgen05 kernel (G4_PREFILL_TC=0 keeps them on the mma.sync
-// kernels below, for A/B runs and for tests that compare the two).
+// Chunks of 64 rows or more run on the tcgen05 kernel; the mma.sync kernels below take shorter ones, an output
+// that is not 16-byte aligned and, with G4_PREFILL_TC=0, everything (A/B runs, tests that compare the two).
 int attn_prefill_flash(const char* fn, const uint16_t* d_q, float scale, int Hq, int Hk, int base_pos, int rows,
                        int stride, uint16_t* d_out, const int8_t* d_ck, const int8_t* d_cv, const float* d_ks,
                        const float* d_vs, const int* d_pt) {
   const char* tc_env = std::getenv("G4_PREFILL_TC");
-  if (rows >= 64 && !(tc_env != nullptr && tc_env[0] == '0')) {
+  if (rows >= 64 && aligned16(d_out) && !(tc_env != nullptr && tc_env[0] == '0')) {
     const int rc = attn_prefill_tc(fn, d_q, scale, Hq, Hk, base_pos, rows, stride, d_out, d_ck, d_cv, d_ks, d_vs, d_pt);
     if (rc <= 0) return rc;
   }

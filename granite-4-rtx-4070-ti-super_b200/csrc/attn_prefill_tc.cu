@@ -17,6 +17,12 @@
 //                   operand)
 // so that one K / V tile, converted from int8 ONCE, serves 256 query rows.
 //
+// A short chunk after a long prefix has few such CTAs (rows / 64 x kv heads), each with a long walk. The
+// cache range of a block is then split over the CTAs of a thread-block cluster (plan_splits): each walks
+// its share of the tiles with its own softmax state, and the partial O rows meet in distributed shared
+// memory as a reduce-scatter - rank o finishes a contiguous part of the 256 rows - so that no workspace
+// in global memory and no second launch are needed. PLACEHOLDER_MEASURED
+//
 // Roles by warp (14 warps; every hand-over is an mbarrier, every wait on one is bounded):
 //   warp 0      producer: looks the tile's 64 positions up in the page table and fetches their raw
 //               K and V code rows with bulk asynchronous copies (TMA engine, cp.async.bulk into this
@@ -49,6 +55,7 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <atomic>
 #include <climits>
 #include <cmath>
@@ -105,9 +112,20 @@ struct TcParams {
   uint16_t* out;
   unsigned int* status;
   int rows, base_pos, Hq, Hk;
+  int splits;  // CTAs of a cluster that share a block's cache range
   long long stride;
   float scale_log2;
 };
+
+// What a split block's CTAs send each other lies over the operand tiles, which nobody reads any more by then:
+// partial O as [sender][16-byte chunk of the row][row of the receiver], so that the lanes of a warp write and read
+// consecutive addresses, then {maximum, sum} as [sender][row].
+constexpr int kMaxSplits = 16;
+constexpr int kRows = 128 * kRowTiles;
+constexpr uint32_t kRecvMl = (kRows + kMaxSplits) * kD * 4;
+static_assert(kRecvMl + (kRows + kMaxSplits) * 8 <= kRowTiles * kQTileBytes + 2 * kBufs * kKvTileBytes,
+              "the exchange fits into the operand tiles");
+__host__ __device__ constexpr int rows_per_rank(int splits) { return (kRows + splits - 1) / splits; }
 
 // tensor-memory columns: S[t][buffer] 64 each, then O[t] 128 each
 constexpr uint32_t kTmemCols = 512;
@@ -145,6 +163,14 @@ __device__ __forceinline__ bool wait_tc(uint64_t* bar, uint32_t parity, TcSmem* 
   *ab = 1;
   if (status != nullptr) atomicOr(status, kStatusAttnWaitTimeout);
   return false;
+}
+
+// Phase of the hardware cluster barrier; every thread of every CTA of the cluster calls it equally often.
+__device__ __forceinline__ void cluster_phase() {
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+__device__ __forceinline__ void store_cluster16(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
 }
 
 __device__ __forceinline__ float ex2_approx(float x) {
@@ -201,12 +227,23 @@ __global__ void __launch_bounds__(kThreads, 1) attn_prefill_tc_kernel(const TcPa
   TcSmem* sm = reinterpret_cast<TcSmem*>(smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u));
   const int warp = warp_index(), lane = threadIdx.x & 31;
   const int hkv = blockIdx.y;
+  // a cluster is p.splits consecutive CTAs along x, so this is the rank in it
+  const int splits = p.splits, rank = static_cast<int>(blockIdx.x) % splits;
   // the longest prefixes first
-  const int blk = static_cast<int>(gridDim.x) - 1 - static_cast<int>(blockIdx.x);
+  const int blk = (static_cast<int>(gridDim.x) - 1 - static_cast<int>(blockIdx.x)) / splits;
   const int row0 = blk * kCtaPos;                           // first chunk row of this CTA
   const int nrows = min(kCtaPos, p.rows - row0);            // its live rows
   const int kv_end = p.base_pos + row0 + nrows;             // cache positions [0, kv_end) are needed
-  const int n_kv = (kv_end + kTN - 1) / kTN;
+  const int n_all = (kv_end + kTN - 1) / kTN;
+  const int tile0 = static_cast<int>(1ll * n_all * rank / splits);                   // this CTA's tiles of the cache:
+  const int share = static_cast<int>(1ll * n_all * (rank + 1) / splits) - tile0;     // tile0 .. tile0 + share - 1 (may be none)
+  // A share that does not begin with tile 0 looks at that tile's logits first, without its P V: the first
+  // tile sets the maximum that a row's probabilities are taken against, so they round to f16 as in the unsplit
+  // walk, and the split changes the order of f32 additions only.
+  const int probe = tile0 > 0 && share > 0 ? 1 : 0;
+  const int n_kv = share + probe;  // tiles walked
+  auto tile_at = [&](int j) { return j < probe ? 0 : tile0 + j - probe; };
+  const int row_tiles = nrows > kQPos ? 2 : 1;              // a row tile without a live row has no work
   const size_t head_row0 = static_cast<size_t>(hkv) * p.stride;
 
   if (threadIdx.x == 0) {
@@ -239,7 +276,8 @@ __global__ void __launch_bounds__(kThreads, 1) attn_prefill_tc_kernel(const TcPa
     // ---- producer ---------------------------------------------------------------------------
     // lane l fetches positions l and l + 32 of every tile
     auto rows_of = [&](int j, int& a, int& b) {
-      const int pa = min(j * kTN + lane, kv_end - 1), pb = min(j * kTN + 32 + lane, kv_end - 1);  // past the end: a row that is masked anyway
+      const int first = tile_at(j) * kTN;
+      const int pa = min(first + lane, kv_end - 1), pb = min(first + 32 + lane, kv_end - 1);  // past the end: a row that is masked anyway
       a = p.pt != nullptr ? __ldg(p.pt + pa) : pa;
       b = p.pt != nullptr ? __ldg(p.pt + pb) : pb;
       a = min(max(a, 0), static_cast<int>(p.stride) - 1), b = min(max(b, 0), static_cast<int>(p.stride) - 1);
@@ -294,8 +332,9 @@ __global__ void __launch_bounds__(kThreads, 1) attn_prefill_tc_kernel(const TcPa
     // uniform registers. With the loop under `if (lane == 0)` an MMA held the thread for ~45 ns, 24 of them
     // most of a tile's 1.85 us: a prefill chunk of 1999 rows after 30000 positions took 1675 us, 1400 now, 8192 rows from 0 906 and 760.
     bool ok = wait_tc(&sm->q_ready, 0, sm, p.status);
-    const uint32_t q_lo = (smem_u32(sm->q16[0]) >> 4) | (1u << 16), k_lo = (smem_u32(sm->k16[0]) >> 4) | (1u << 16);
-    const uint32_t v_lo = (smem_u32(sm->v16[0]) >> 4) | ((kKvTileBytes / 2 >> 4) << 16);  // 64-dim halves 8 KB apart
+    // (the address field has 14 bits; in a cluster the rank stands in the bits above and would run into the offset)
+    const uint32_t q_lo = ((smem_u32(sm->q16[0]) >> 4) & 0x3fffu) | (1u << 16), k_lo = ((smem_u32(sm->k16[0]) >> 4) & 0x3fffu) | (1u << 16);
+    const uint32_t v_lo = ((smem_u32(sm->v16[0]) >> 4) & 0x3fffu) | ((kKvTileBytes / 2 >> 4) << 16);  // 64-dim halves 8 KB apart
     auto issue_s = [&](int j) {
       const int b = j % kBufs, sb = j & 1;
       if (!(ok = ok && wait_tc(&sm->kv_full[b], (j / kBufs) & 1, sm, p.status))) return;
@@ -303,6 +342,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_prefill_tc_kernel(const TcPa
       if (elect_one()) {
 #pragma unroll
         for (int t = 0; t < kRowTiles; ++t) {
+          if (t >= row_tiles) break;
 #pragma unroll
           for (int kk = 0; kk < 8; ++kk)  // 16 dims = 32 bytes per instruction; dims 64.. in the second half tile
             mma_f16_ss(tmem_base + s_col(t, sb), desc_of(q_lo + ((t * kQTileBytes + (kk >> 2) * (kQTileBytes / 2) + (kk & 3) * 32) >> 4)),
@@ -312,18 +352,20 @@ __global__ void __launch_bounds__(kThreads, 1) attn_prefill_tc_kernel(const TcPa
       }
       __syncwarp();
     };
-    if (ok) issue_s(0);
+    if (ok && n_kv > 0) issue_s(0);
     for (int j = 0; j < n_kv && ok; ++j) {
       if (j + 1 < n_kv) issue_s(j + 1);
       const int b = j % kBufs, sb = j & 1;
-      for (int t = 0; t < kRowTiles && ok; ++t) {
+      for (int t = 0; t < row_tiles && ok; ++t) {
         if (!(ok = wait_tc(&sm->p_full[t][sb], (j >> 1) & 1, sm, p.status))) break;
         tc_fence_after();
         if (elect_one()) {
+          if (j >= probe) {
 #pragma unroll
-          for (int kk = 0; kk < 4; ++kk)  // 16 positions per instruction: 8 columns of P, two 8-row groups of V
-            mma_f16_ts(tmem_base + o_col(t), tmem_base + s_col(t, sb) + kk * 8, desc_of(v_lo + ((b * kKvTileBytes + kk * 2048) >> 4)),
-                       kIdescPV, (j > 0 || kk > 0) ? 1u : 0u);
+            for (int kk = 0; kk < 4; ++kk)  // 16 positions per instruction: 8 columns of P, two 8-row groups of V
+              mma_f16_ts(tmem_base + o_col(t), tmem_base + s_col(t, sb) + kk * 8, desc_of(v_lo + ((b * kKvTileBytes + kk * 2048) >> 4)),
+                         kIdescPV, (j > probe || kk > 0) ? 1u : 0u);
+          }
           mma_commit<false>(smem_u32(&sm->pv_done[t][sb]));
         }
         __syncwarp();
@@ -425,11 +467,12 @@ __global__ void __launch_bounds__(kThreads, 1) attn_prefill_tc_kernel(const TcPa
     // finite maximum: all its logits are masked and it never looks for one.
     float m_run = live ? -INFINITY : 0.0f, l_run = 0.0f;
     bool ok = true;
-    for (int j = 0; j < n_kv; ++j) {
+    const int n_mine = t < row_tiles ? n_kv : 0;
+    for (int j = 0; j < n_mine; ++j) {
       const int sb = j & 1, b = j % kBufs;
       if (!(ok = wait_tc(&sm->s_full[t][sb], (j >> 1) & 1, sm, p.status))) break;
       tc_fence_after();
-      const int kv0 = j * kTN;
+      const int kv0 = tile_at(j) * kTN;
       const uint32_t s_addr = lane_addr + s_col(t, sb);
       // only a tile that reaches past the warp's first position needs the causal mask (warp-uniform)
       const bool masked = !all_live || kv0 + kTN - 1 > pos_first;
@@ -479,7 +522,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_prefill_tc_kernel(const TcPa
         const float corr = (grow && m_run > -INFINITY) ? ex2_approx(m_run - m_new) : 1.0f;
         l_run *= corr;
         m_run = m_new;
-        if (j > 0) {
+        if (j > probe) {
           // O has to shrink: it is complete (and nobody adds to it) once the previous tile's P V is done
           if (!(ok = wait_tc(&sm->pv_done[t][(j - 1) & 1], ((j - 1) >> 1) & 1, sm, p.status))) break;
           tc_fence_after();
@@ -495,6 +538,12 @@ __global__ void __launch_bounds__(kThreads, 1) attn_prefill_tc_kernel(const TcPa
         }
       }
       if (!ok) break;
+      if (j < probe) {  // the maximum was all there was to learn
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(smem_u32(&sm->p_full[t][sb]));
+        continue;
+      }
       l_run += l_tile;
       // The probabilities go over the first 32 columns of the logits they came from. That buffer last
       // held P of tile j - 2, and S of tile j, issued after that tile's P V, has completed: MMAs
@@ -507,10 +556,65 @@ __global__ void __launch_bounds__(kThreads, 1) attn_prefill_tc_kernel(const TcPa
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&sm->p_full[t][sb]));
     }
-    // ---- the finished row: O / l -> bf16
-    if (ok && n_kv > 0) ok = wait_tc(&sm->pv_done[t][(n_kv - 1) & 1], ((n_kv - 1) >> 1) & 1, sm, p.status);
-    if (ok) {
-      tc_fence_after();
+    if (ok && n_mine > 0) ok = wait_tc(&sm->pv_done[t][(n_mine - 1) & 1], ((n_mine - 1) >> 1) & 1, sm, p.status);
+    tc_fence_after();
+    __syncwarp();
+    if (splits > 1) {
+      // ---- a share of the cache: the partial row goes to the rank that finishes it
+      const int per = rows_per_rank(splits), mine = t * 128 + r;
+      const int owner = mine / per, local = mine - owner * per;
+      cluster_phase();  // every CTA of the cluster runs and is done with its operand tiles
+      const uint32_t base = cluster_addr(smem_u32(sm), static_cast<uint32_t>(owner));
+#pragma unroll 1
+      for (int oc = 0; oc < 4; ++oc) {
+        uint32_t v[32];
+        __syncwarp();
+        if (n_mine > 0) {
+          tmem_ld32(lane_addr + o_col(t) + oc * 32, v);
+          tmem_ld_wait();
+        } else {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) v[i] = 0u;
+        }
+        if (live) {
+#pragma unroll
+          for (int i = 0; i < 32; i += 4)
+            store_cluster16(base + static_cast<uint32_t>((rank * 32 + oc * 8 + i / 4) * per + local) * 16, v[i], v[i + 1], v[i + 2],
+                            v[i + 3]);
+        }
+      }
+      if (live)
+        asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(base + kRecvMl + static_cast<uint32_t>(rank * per + local) * 8),
+                     "f"(m_run), "f"(l_run)
+                     : "memory");
+      cluster_phase();  // every partial row has arrived
+      // ---- this rank's rows: sum of the shares in rank order, each scaled to the common maximum
+      const float4* got = reinterpret_cast<const float4*>(sm);
+      const float2* ml = reinterpret_cast<const float2*>(reinterpret_cast<const uint8_t*>(sm) + kRecvMl);
+      for (int i = static_cast<int>(threadIdx.x) - 128; i < per * 16; i += 256) {
+        const int lr = i % per, c = i / per, row = rank * per + lr;  // eight dims of one row
+        const int tr = row >> 7, out_row = row0 + tr * kQPos + (row & 31), head = hkv * 4 + ((row >> 5) & 3);
+        if (row >= kRows || out_row >= p.rows) continue;
+        float m = -INFINITY;
+        for (int q = 0; q < splits; ++q) m = fmaxf(m, ml[q * per + lr].x);
+        float l = 0.0f, o[8] = {};
+        for (int q = 0; q < splits; ++q) {
+          const float2 e = ml[q * per + lr];
+          // a share without a live logit has sum and O zero (or NaN, which has to stay)
+          const float w = e.x == -INFINITY ? 0.0f : ex2_approx(e.x - m);
+          const float4 x = got[(q * 32 + 2 * c) * per + lr], y = got[(q * 32 + 2 * c + 1) * per + lr];
+          l += e.y * w;
+          o[0] += x.x * w, o[1] += x.y * w, o[2] += x.z * w, o[3] += x.w * w;
+          o[4] += y.x * w, o[5] += y.y * w, o[6] += y.z * w, o[7] += y.w * w;
+        }
+        const float inv = l > 0.0f ? 1.0f / l : 0.0f;
+        uint4 u;
+        u.x = pack_bf16x2(o[0] * inv, o[1] * inv), u.y = pack_bf16x2(o[2] * inv, o[3] * inv);
+        u.z = pack_bf16x2(o[4] * inv, o[5] * inv), u.w = pack_bf16x2(o[6] * inv, o[7] * inv);
+        *reinterpret_cast<uint4*>(p.out + (static_cast<size_t>(out_row) * p.Hq + head) * kD + c * 8) = u;
+      }
+    } else if (ok && n_mine > 0) {
+      // ---- the finished row: O / l -> bf16
       const float inv = l_run > 0.0f ? 1.0f / l_run : 0.0f;
       uint16_t* dst = p.out + (static_cast<size_t>(live ? crow : 0) * p.Hq + hkv * 4 + hl) * kD;
 #pragma unroll 1
@@ -531,6 +635,11 @@ __global__ void __launch_bounds__(kThreads, 1) attn_prefill_tc_kernel(const TcPa
         }
       }
     }
+  }
+  if (splits > 1 && (warp < 4 || warp >= 12)) {  // the two phases of the exchange
+    __syncwarp();
+    cluster_phase();
+    cluster_phase();
   }
 
   // Wind down. On the normal path every softmax thread has seen the last P V complete and every
@@ -553,6 +662,65 @@ __global__ void __launch_bounds__(kThreads, 1) attn_prefill_tc_kernel(const TcPa
 
 }  // namespace
 
+// CTAs of one cluster size that the current device runs at once (0: none, or the query failed); asked once
+// per device and size.
+static int resident_ctas(int splits) {
+  static std::atomic<int> known[64][kMaxSplits + 1];  // 1 + the answer
+  int dev = -1;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0) return 0;
+  if (dev < 64)
+    if (const int k = known[dev][splits].load(std::memory_order_relaxed); k != 0) return k - 1;
+  int n = 0;
+  if (splits == 1) {
+    n = sm_count();
+  } else if (splits <= 8 || cudaFuncSetAttribute(attn_prefill_tc_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
+                                cudaSuccess) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(static_cast<unsigned>(splits)), cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = kTcSmemBytes;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = static_cast<unsigned>(splits), attr[0].val.clusterDim.y = 1, attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr, cfg.numAttrs = 1;
+    if (cudaOccupancyMaxActiveClusters(&n, attn_prefill_tc_kernel, &cfg) != cudaSuccess) n = 0;
+    n *= splits;
+  }
+  (void)cudaGetLastError();
+  if (dev < 64) known[dev][splits].store(n + 1, std::memory_order_relaxed);
+  return n;
+}
+
+// CTAs per block of query positions. The cost of a plan in cache tiles (~1.3 us): the blocks go over the SMs in
+// rounds, the longest prefixes first, and a round takes its longest block's share plus what a CTA costs beside
+// its tiles (Q rows, first pages, the last P V: kFixed; the look at tile 0 and the exchange: kExchange). Fewer
+// CTAs win a tie. From four rounds on the rounds are full enough and nothing is split. Large clusters lose by
+// themselves: few of them fit between the chip's SM clusters. G4_PREFILL_SPLITS forces a count (tests,
+// measurements). PLACEHOLDER_PLAN
+static int plan_splits(int rows, int base_pos, int Hk) {
+  constexpr double kFixed = 3.0, kExchange = 3.0;
+  if (const char* v = std::getenv("G4_PREFILL_SPLITS"); v != nullptr && std::atoi(v) > 0) {
+    const int s = std::min(std::atoi(v), kMaxSplits);
+    return resident_ctas(s) > 0 ? s : 1;
+  }
+  const int blocks = (rows + kCtaPos - 1) / kCtaPos, sms = sm_count();
+  const long long units = 1ll * blocks * Hk;
+  if (units >= 4ll * sms) return 1;
+  int best = 1;
+  double least = 1e300;
+  for (int s = 1; s <= kMaxSplits; ++s) {
+    const int per_round = resident_ctas(s) / s;  // blocks
+    if (per_round <= 0) continue;
+    double cost = 0.0;
+    for (long long u = 0; u < units; u += per_round) {
+      const int blk = blocks - 1 - static_cast<int>(u / Hk);
+      const int tiles = (base_pos + std::min(rows, (blk + 1) * kCtaPos) + kTN - 1) / kTN;
+      cost += (tiles + s - 1) / s + kFixed + (s > 1 ? kExchange : 0.0);
+    }
+    if (cost < least * 0.98) least = cost, best = s;
+  }
+  return best;
+}
+
 // Launch for a chunk of at least 64 rows; arguments as granite4_prefill_attention_int8 (validated
 // there). Returns 1 when the device status word cannot be resolved (the caller then takes the
 // mma.sync form), 0 on success, -1 on a launch error.
@@ -573,8 +741,22 @@ int attn_prefill_tc(const char* fn, const uint16_t* d_q, float scale, int Hq, in
   p.q = d_q, p.ck = d_ck, p.cv = d_cv, p.ks = d_ks, p.vs = d_vs, p.pt = d_pt, p.out = d_out, p.status = status;
   p.rows = rows, p.base_pos = base_pos, p.Hq = Hq, p.Hk = Hk, p.stride = stride;
   p.scale_log2 = scale * 1.4426950408889634f;
-  const dim3 grid(static_cast<unsigned>((rows + kCtaPos - 1) / kCtaPos), static_cast<unsigned>(Hk));
-  G4_LAUNCH_PDL(fn, attn_prefill_tc_kernel, grid, dim3(kThreads), kTcSmemBytes, current_stream(), p);
+  p.splits = plan_splits(rows, base_pos, Hk);
+  const dim3 grid(static_cast<unsigned>((rows + kCtaPos - 1) / kCtaPos * p.splits), static_cast<unsigned>(Hk));
+  if (p.splits == 1) {
+    G4_LAUNCH_PDL(fn, attn_prefill_tc_kernel, grid, dim3(kThreads), kTcSmemBytes, current_stream(), p);
+    return 0;
+  }
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid, cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = kTcSmemBytes, cfg.stream = current_stream();
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = static_cast<unsigned>(p.splits), attr[0].val.clusterDim.y = 1, attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr, cfg.numAttrs = pdl_enabled() ? 2u : 1u;
+  G4_CUDA_TRY(fn, cudaLaunchKernelEx(&cfg, attn_prefill_tc_kernel, p));
   return 0;
 }
 

@@ -145,3 +145,42 @@ def test_a_query_head_that_is_not_a_number_stays_in_its_rows(K):
     keep = np.ones((rows, Hq), bool)
     keep[70, 5] = False
     assert close(f32_of(got[keep]), f32_of(clean[keep]), 0.0)  # (when a maximum moves may differ within the warp)
+
+
+@pytest.mark.parametrize("rows,base,splits,sigma", [(64, 0, 16, 1.0), (65, 700, 8, 2.0), (64, 64, 3, 2.0), (100, 37, 5, 60.0),
+                                                    (200, 1000, 2, 2.0), (96, 1900, 16, 60.0), (65, 1983, 7, 1.0)])
+def test_cache_range_split_over_a_cluster(K, monkeypatch, rows, base, splits, sigma):
+    """The cache range of a block split over a cluster: shares without a tile, row counts of the exchange
+    that do not divide 256, a row tile without a live row, and magnitudes at which the shares' maxima lie
+    far apart; against float64, and against the unsplit walk: where no later tile moves the maximum that tile 0 set
+    (by 2^12, sigma below 10) only the order of f32 additions differs, at most one bf16 step in a few elements."""
+    stride = 2048
+    pl = pool(rows + splits, stride)
+    rng = np.random.default_rng(rows * 5 + base)
+    table = rng.permutation(stride).astype(np.int32)
+    q = bf16_bits(sigma * rng.standard_normal((rows, Hq * D)))
+    monkeypatch.setenv("G4_PREFILL_SPLITS", str(splits))
+    got = run(K, q, pl, base, stride, table)
+    monkeypatch.setenv("G4_PREFILL_SPLITS", "1")
+    whole = run(K, q, pl, base, stride, table)
+    tol = 0.02 if sigma > 10 else 0.01  # the bars of the unsplit form above
+    assert close(f32_of(got), f32_of(whole), tol / 4)
+    # f32 sums in another order differ by some 1e-6 relative, 2^-8 is a bf16 step: about one element in 2000 rounds apart
+    assert sigma > 10 or (got != whole).mean() < 5e-3
+    sel = np.unique(np.r_[0:3, 30:34, rows // 2, rows - 2:rows]).astype(int)
+    sel = sel[sel < rows]
+    exact = f64_rows(q[sel], pl, [table] * len(sel), (base + sel).astype(np.int32))
+    assert close(f32_of(got[sel]).reshape(len(sel), Hq, D), exact, tol)
+
+
+def test_output_that_is_not_16_byte_aligned(K):
+    """An output on a 4-byte boundary is taken by the kernels that store four bytes at a time."""
+    rows, stride = 64, 128
+    pl = pool(3, stride)
+    q = bf16_bits(np.random.default_rng(4).standard_normal((rows, Hq * D)))
+    want = run(K, q, pl, 0, stride, None)
+    buf = torch.zeros(rows * Hq * D + 8, dtype=torch.int16, device=DEV)
+    out = buf[2:2 + rows * Hq * D].view(rows, Hq * D)
+    assert K.prefill_attention_int8(dev(q), SCALE, Hq, Hk, D, 0, stride, out, *[dev(x) for x in pl], pt=None) == 0
+    got = out.cpu().numpy().view(np.uint16)
+    assert close(f32_of(got), f32_of(want), 0.01) and int(buf[:2].abs().sum()) == 0 and int(buf[-6:].abs().sum()) == 0
