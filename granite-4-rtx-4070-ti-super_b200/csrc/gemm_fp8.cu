@@ -32,6 +32,7 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 #include <cstdlib>
 #include <map>
@@ -279,8 +280,9 @@ __device__ __forceinline__ void store4(const GemmParams& p, float4 v, int row, i
 // Fused SwiGLU epilogue of one warp's 32 rows: gate from the first `half` columns of the accumulator and
 // up from the next, a = bf16(silu(g) u) (the arithmetic of the standalone kernel, g4_math.cuh swiglu) for
 // output columns n0 .. n0 + half - 1, and the running max |a| of what was stored (packed bf16 pairs).
+// up_at: accumulator column where the up half starts.
 __device__ __forceinline__ uint32_t store_accumulator_swiglu(const GemmParams& p, uint32_t taddr, int row, int n0,
-                                                             float a_scale, int half) {
+                                                             float a_scale, int half, int up_at) {
   uint32_t amax = 0u;
   const int I = p.swiglu_i;
 #pragma unroll 1
@@ -290,7 +292,7 @@ __device__ __forceinline__ uint32_t store_accumulator_swiglu(const GemmParams& p
     uint32_t gv[32], uv[32];
     __syncwarp();
     tmem_ld32(taddr + c * 32, gv);
-    tmem_ld32(taddr + half + c * 32, uv);
+    tmem_ld32(taddr + up_at + c * 32, uv);
     tmem_ld_wait();
     if (row >= p.M) continue;
     const bool one_scale = (n >= p.seg1 || n + 32 <= p.seg1) && (n >= p.seg2 || n + 32 <= p.seg2) &&
@@ -645,7 +647,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         if (slabs)
           amax = store_slabs(p, &map_out, &map_res, st, ring, taddr, lane, row0, n0, n_end, bn / 2, a_scale, ok);
         else if (p.swiglu_i)
-          amax = store_accumulator_swiglu(p, taddr, row0 + lane, n0, a_scale, bn / 2);
+          amax = store_accumulator_swiglu(p, taddr, row0 + lane, n0, a_scale, bn / 2, bn / 2);
         else
           store_accumulator(p, taddr, row0 + lane, n0, bn, a_scale, partial != nullptr ? partial + size_t(q * 32 + lane) * kBN : nullptr);
         if (p.swiglu_i) {
@@ -726,9 +728,13 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
 // because one thread gets through only about three loads per microsecond and a 32-column block is
 // just 4 KB. The MMA thread issues 4 p.kc MMAs (M 128, N p.bn, K 32) per stage; an MMA of up to 32
 // columns takes ~46 cycles (measured; 64 -> 48, 128 -> 64, 256 -> 128), so a 32-column tile
-// consumes 22 weight bytes per cycle, just under an SM's share of HBM. p.a_rows = 16 fetches only
-// 16 rows of A per block (the MMA reads 128 rows of shared memory wherever the 16 end: rows of D
-// nobody reads). Roles, barriers and the bounded waits are those of gemm_fp8_kernel.
+// consumes 22 weight bytes per cycle, just under an SM's share of HBM. Only p.a_rows rows of A, M rounded
+// up to 16, are fetched per block (the MMA reads 128 rows of shared memory wherever they end: rows of D
+// nobody reads): every CTA reads all of A, so that with a 32-column tile four of five bytes it fetched
+// were A when the block was always 128 rows. PLACEHOLDER_STREAM
+// Fused SwiGLU: a tile is p.bn / 2 gate rows and as many up rows of W, two MMAs per 32 bytes of K, gate in
+// accumulator columns 0 .. and up from column 128.
+// Roles, barriers and the bounded waits are those of gemm_fp8_kernel.
 constexpr int kStreamMaxStages = 8;
 struct StreamRing {
   uint64_t full[kStreamMaxStages], empty[kStreamMaxStages], acc_full[kAccs], acc_empty[kAccs];
@@ -758,7 +764,9 @@ gemm_fp8_stream_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
   const uint32_t tiles_addr = (raw + 1023u) & ~1023u;
   StreamRing* ring = reinterpret_cast<StreamRing*>(smem_raw + (tiles_addr - raw) + kStreamTileBytes + (kBM - 16) * kBK);
   const int warp = warp_index(), lane = threadIdx.x & 31;
-  const uint32_t a_blk = uint32_t(p.a_rows) * kBK, w_blk = uint32_t(p.bn) * kBK;
+  // W comes as one part of p.bn rows per k-block, or as gate rows and up rows of half as many
+  const int parts = p.swiglu_i ? 2 : 1, w_rows = p.bn / parts, n_out = p.swiglu_i ? p.swiglu_i : p.N;
+  const uint32_t a_blk = uint32_t(p.a_rows) * kBK, w_blk = uint32_t(p.bn) * kBK, part_blk = uint32_t(w_rows) * kBK;
   const uint32_t stage_bytes = uint32_t(p.kc) * (a_blk + w_blk);
 
   if (threadIdx.x == 0) {
@@ -779,7 +787,7 @@ gemm_fp8_stream_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if (warp != 0) pdl_begin();
 
-  const int tiles = (p.N + p.bn - 1) / p.bn, kblocks = (p.K + kBK - 1) / kBK;
+  const int tiles = (n_out + w_rows - 1) / w_rows, kblocks = (p.K + kBK - 1) / kBK;
   const int stages_per_tile = (kblocks + p.kc - 1) / p.kc;
 
   if (warp == 0) {
@@ -794,11 +802,15 @@ gemm_fp8_stream_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
       if (p.box3d) {  // one box per operand and stage; k-blocks past K are filled with zeros
         if (lane == 0) {
           if (load_a) tma_load_3d(dst, &map_a, 0, 0, kb, bar);
-          if (load_w) tma_load_3d(dst + p.kc * a_blk, &map_w, 0, t * p.bn, kb, bar);
+          if (load_w)
+            for (int h = 0; h < parts; ++h)
+              tma_load_3d(dst + p.kc * (a_blk + h * part_blk), &map_w, 0, h * n_out + t * w_rows, kb, bar);
         }
       } else if (lane < nblk) {
         if (load_a) tma_load_2d<false>(dst + lane * a_blk, &map_a, kb * kBK, 0, bar);
-        if (load_w) tma_load_2d<false>(dst + p.kc * a_blk + lane * w_blk, &map_w, kb * kBK, t * p.bn, bar);
+        if (load_w)
+          for (int h = 0; h < parts; ++h)
+            tma_load_2d<false>(dst + p.kc * (a_blk + h * part_blk) + lane * part_blk, &map_w, kb * kBK, h * n_out + t * w_rows, bar);
       }
       return nblk;
     };
@@ -826,7 +838,7 @@ gemm_fp8_stream_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
       issue(it, true, true);
     }
   } else if (warp == 1) {
-    const uint32_t idesc = (1u << 4) | (uint32_t(p.bn >> 3) << 17) | (uint32_t(kBM >> 4) << 24);
+    const uint32_t idesc = (1u << 4) | (uint32_t(w_rows >> 3) << 17) | (uint32_t(kBM >> 4) << 24);
     uint32_t s = 0, ph = 0, local = 0;
     bool ok = true;
     for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x, ++local) {
@@ -841,10 +853,13 @@ gemm_fp8_stream_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
         const int nblk = min(p.kc, kblocks - st * p.kc);
         if (elect_one()) {
           for (int j = 0; j < nblk; ++j) {
-            const uint64_t a_desc = smem_desc_k128(base + j * a_blk), w_desc = smem_desc_k128(base + p.kc * a_blk + j * w_blk);
+            const uint64_t a_desc = smem_desc_k128(base + j * a_blk);
+            for (int h = 0; h < parts; ++h) {
+              const uint64_t w_desc = smem_desc_k128(base + p.kc * (a_blk + h * part_blk) + j * part_blk);
 #pragma unroll
-            for (int k = 0; k < kBK / 32; ++k)
-              mma_f8<false>(d_tmem, a_desc + uint64_t(2 * k), w_desc + uint64_t(2 * k), idesc, (st | j | k) != 0);
+              for (int k = 0; k < kBK / 32; ++k)
+                mma_f8<false>(d_tmem + h * (kBN / 2), a_desc + uint64_t(2 * k), w_desc + uint64_t(2 * k), idesc, (st | j | k) != 0);
+            }
           }
           mma_commit<false>(smem_u32(&ring->empty[s]));
         }
@@ -861,11 +876,16 @@ gemm_fp8_stream_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
     bool ok = true;
     for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x, ++local) {
       const uint32_t acc = local & 1u, aph = (local >> 1) & 1u;
-      const int n0 = t * p.bn, n_end = min(p.N, n0 + p.bn), row = q * 32 + lane;
+      const int n0 = t * w_rows, n_end = min(n_out, n0 + w_rows), row = q * 32 + lane;
       if (!(ok = stream_wait(&ring->acc_full[acc], aph, ring, p.status))) break;
       tc_fence_after();
-      if (q * 32 < p.M) {  // uniform over the warp
-        const uint32_t taddr = tmem_base + (uint32_t(q * 32) << 16) + acc * kBN;
+      const uint32_t taddr = tmem_base + (uint32_t(q * 32) << 16) + acc * kBN;
+      if (p.swiglu_i && q * 32 < p.M) {
+        uint32_t amax = store_accumulator_swiglu(p, taddr, row, n0, a_scale, w_rows, kBN / 2);
+        __syncwarp();
+        amax = amax_warp(amax);
+        if (lane == 0 && amax != 0u) atomic_amax(p.amax_slot + 1, amax_value(amax));
+      } else if (q * 32 < p.M) {  // uniform over the warp
 #pragma unroll 1
         for (int c = 0; n0 + c * 32 < n_end; ++c) {
           uint32_t v[32];
@@ -1361,21 +1381,23 @@ SplitPlan plan_split(int M, int N, int K, int sms) {
 }
 
 // Tile width and ring shape of the stream form. A round of tiles over `sms` CTAs costs what its
-// slowest resource costs: the MMA thread (4 MMAs per k-block at ~max(46, bn / 2) cycles) or the SM's
-// share of HBM (bn x K bytes at ~44 bytes per ns); the plan is the width with the cheapest total.
-// Ties go to the wider tile (fewer A blocks and loader steps per weight byte).
+// slowest resource costs: the MMA thread (4 MMAs per k-block at ~max(46, bn / 2) cycles), the SM's
+// share of HBM (bn x K bytes at ~44 bytes per ns) or what one CTA fetches through L2 (A and W at ~60
+// bytes per ns); the plan is the width with the cheapest total. Ties go to the wider tile (fewer A
+// blocks and loader steps per weight byte). swiglu: the width is half gate, half up rows and the
+// epilogue works in chunks of 32 output columns; N is then the number of output columns.
 struct StreamPlan {
   int bn, kc, stages;
 };
-StreamPlan plan_stream(int N, int K, int a_rows, int sms) {
-  const int kblocks = (K + kBK - 1) / kBK;
+StreamPlan plan_stream(int N, int K, int a_rows, int sms, bool swiglu) {
+  const int kblocks = (K + kBK - 1) / kBK, parts = swiglu ? 2 : 1;
   double best = 1e300;
   StreamPlan pl{kBN, 1, 4};
-  for (int bn = 32; bn <= kBN; bn += 16) {
-    const int tiles = (N + bn - 1) / bn, rounds = (tiles + sms - 1) / sms;
-    const double mma_ns = 4.0 * kblocks * (bn / 2 > 46 ? bn / 2 : 46) / 1.85;
-    const double hbm_ns = double(bn) * K / 44.0;
-    const double cost = rounds * (mma_ns > hbm_ns ? mma_ns : hbm_ns) + 500.0 * rounds;
+  for (int w = 32; w * parts <= kBN; w += swiglu ? 32 : 16) {
+    const int bn = w * parts, tiles = (N + w - 1) / w, rounds = (tiles + sms - 1) / sms;
+    const double mma_ns = 4.0 * parts * kblocks * (w / 2 > 46 ? w / 2 : 46) / 1.85;
+    const double hbm_ns = double(bn) * K / 44.0, fetch_ns = double(bn + a_rows) * K / 60.0;
+    const double cost = rounds * std::max(mma_ns, std::max(hbm_ns, fetch_ns)) + 500.0 * rounds;
     if (cost <= best * 1.0001) best = cost, pl.bn = bn;
   }
   const int blk = (a_rows + pl.bn) * kBK;  // bytes of one k-block of a stage
@@ -1401,13 +1423,15 @@ bool make_map3d(CUtensorMap* map, const void* base, int rows, int K, long long l
 }
 
 int launch_stream(const char* fn, const uint8_t* d_a, long long lda, const uint8_t* d_w, GemmParams p) {
-  p.a_rows = p.M <= 16 ? 16 : kBM;
-  const StreamPlan pl = plan_stream(p.N, p.K, p.a_rows, sm_count());
+  p.a_rows = (p.M + 15) / 16 * 16;
+  const int n_out = p.swiglu_i ? p.swiglu_i : p.N;
+  const StreamPlan pl = plan_stream(n_out, p.K, p.a_rows, sm_count(), p.swiglu_i != 0);
+  const int w_rows = p.swiglu_i ? pl.bn / 2 : pl.bn;
   p.bn = pl.bn, p.kc = pl.kc, p.stages = pl.stages;
   CUtensorMap map_a, map_w;
   p.box3d = p.K % kBK == 0 && p.kc > 1 && box3d_enabled() && make_map3d(&map_a, d_a, p.M, p.K, lda, p.a_rows, p.kc) &&
-            make_map3d(&map_w, d_w, p.N, p.K, p.K, p.bn, p.kc);
-  if (!p.box3d && (!make_map(&map_a, d_a, p.M, p.K, lda, p.a_rows) || !make_map(&map_w, d_w, p.N, p.K, p.K, p.bn)))
+            make_map3d(&map_w, d_w, p.N, p.K, p.K, w_rows, p.kc);
+  if (!p.box3d && (!make_map(&map_a, d_a, p.M, p.K, lda, p.a_rows) || !make_map(&map_w, d_w, p.N, p.K, p.K, w_rows)))
     return fail(fn, "the tensor map could not be encoded");
   static std::mutex mu;
   static std::map<int, cudaError_t> done;
@@ -1420,7 +1444,7 @@ int launch_stream(const char* fn, const uint8_t* d_a, long long lda, const uint8
                                        int(kStreamSmemBytes));
     G4_CUDA_TRY(fn, done[dev]);
   }
-  const int tiles = (p.N + p.bn - 1) / p.bn;
+  const int tiles = (n_out + w_rows - 1) / w_rows;
   const int grid = tiles < sm_count() ? tiles : sm_count();
   G4_LAUNCH_PDL(fn, gemm_fp8_stream_kernel, dim3(grid), dim3(kThreads), kStreamSmemBytes, current_stream(), map_a,
                 map_w, p);
@@ -1590,7 +1614,8 @@ extern "C" int granite4_kernel_gemm_fp8(int out_kind, const uint8_t* d_a, long l
   if (fused_swiglu) {
     p.swiglu_i = N / 2, p.amax_slot = ep->d_out_scale_amax;
     if (!amax_prezeroed()) G4_CUDA_TRY(fn, cudaMemsetAsync(p.amax_slot, 0, 2 * sizeof(float), current_stream()));
-    if (M <= kBM) return launch<CfgWide>(fn, d_a, lda, d_w, p);  // no split of K under this epilogue
+    // no split of K under this epilogue; the tiled form's 128 output columns leave 48 SMs idle at I = 12800
+    if (M <= kBM) return stream_enabled() ? launch_stream(fn, d_a, lda, d_w, p) : launch<CfgWide>(fn, d_a, lda, d_w, p);
   }
   if (M <= kDecRows && decode_form_enabled()) {
     const int rc = launch_decode(fn, d_a, lda, d_w, p);

@@ -110,3 +110,25 @@ def test_small_norm_quant_and_swiglu_equal_the_oracle(K, port, rows, cols):
     assert np.abs(key(got) - key(want)).max() <= 1  # the stated 1 bf16 ulp
     cs, ss, as_ = port.quant_fp8(got)
     assert (c8.cpu().numpy() == cs).all() and sa[0].item() == ss and sa[1].item() == as_
+
+
+@pytest.mark.parametrize("M,inter,Kd", [(1, 32, 128), (17, 96, 1552), (37, 1000, 512), (64, 12800, 256), (128, 200, 4096)])
+def test_fused_swiglu_of_few_rows_equals_gemm_then_swiglu(K, M, inter, Kd):
+    """Gate and up rows as two parts of one tile: the f32 sums of these integer operands are exact, so the fused
+    epilogue has to give the standalone kernel's bits. Ragged last tiles, K of one block to more than the ring,
+    a K that is not whole blocks."""
+    g = torch.Generator(device=DEV).manual_seed(M * inter + Kd)
+    lut = torch.arange(256, dtype=torch.uint8, device=DEV).view(torch.float8_e4m3fn).float()
+    pick = (lut.abs() <= 2) & (lut == lut.round()) & ~lut.isnan()
+    codes = pick.nonzero().flatten().to(torch.uint8)
+    a = codes[torch.randint(len(codes), (M, Kd), generator=g, device=DEV)].contiguous()
+    w = codes[torch.randint(len(codes), (2 * inter, Kd), generator=g, device=DEV)].contiguous()
+    both = torch.empty(M, 2 * inter, dtype=torch.float32, device=DEV)
+    sc = (2.0 ** -6,)
+    assert K.gemm_fp8(a, w, both, w_scales=sc, workspace=K.gemm_fp8_workspace(M, 2 * inter, Kd, DEV)) == 0
+    assert torch.equal(both, (lut[a.long()].double() @ lut[w.long()].double().T * sc[0]).float())
+    out, slot = torch.empty(M, inter, dtype=torch.bfloat16, device=DEV), torch.full((2,), 9.0, device=DEV)
+    assert K.gemm_fp8(a, w, out, w_scales=sc, swiglu_scale_amax=slot) == 0
+    want, c8, sa = torch.empty_like(out), torch.empty(M, inter, dtype=torch.uint8, device=DEV), torch.zeros(2, device=DEV)
+    assert K.swiglu_fp8(both[:, :inter].contiguous(), both[:, inter:].contiguous(), want, c8, sa) == 0
+    assert torch.equal(out, want) and slot[1].item() == sa[1].item()
