@@ -285,34 +285,35 @@ __global__ void __launch_bounds__(kPfWarps * 32, 3) attn_prefill_kernel(const Pr
   }
 }
 
-// The same with 32 query positions per CTA: every warp owns two 16-row tiles of its head, so a K or V
-// fragment fetched from shared memory feeds four MMAs instead of two and the conversion is shared by 128
-// query rows. The accumulators of two tiles leave no registers for Q and a 64-column S, so Q (fp16) lives
-// in shared memory and a tile of 64 positions is consumed as two halves of 32.
+// The form of a short chunk: a CTA has 32 query positions of ONE query head, four warps = two 16-row tiles x two
+// halves of the 128 output dims. Q (fp16) lives in shared memory and a tile of 64 positions is consumed as two
+// halves of 32. Chunks of 32 - 63 rows walk the whole prefix in a few CTAs, bound by the mma.sync rate of their SMs
+// (~17 cycles per instruction and sub-partition), so the four heads of a kv head take an SM each instead of
+// sharing the conversion of K and V, and two warps compute the same logits to halve P V: 37 rows
+// after 1203 positions 73 us with all four heads in a CTA (two row tiles per warp), 52 now; 63 after 30000 1551 and 1219.
 constexpr int kQRows2 = 32;
+constexpr int kWarps2 = 4;  // warp w: row tile w % 2, output dims 64 (w / 2) ..
 struct PrefillSmem2 {
   PrefillSmem t;
-  __half qh[kPfWarps][kQRows2][kHPitch];
+  __half qh[kQRows2][kHPitch];
 };
 
-__global__ void __launch_bounds__(kPfWarps * 32, 2) attn_prefill2_kernel(const PrefillParams p) {
+__global__ void __launch_bounds__(kWarps2 * 32, 2) attn_prefill2_kernel(const PrefillParams p) {
   extern __shared__ __align__(16) unsigned char pf_smem[];
   PrefillSmem2& sm2 = *reinterpret_cast<PrefillSmem2*>(pf_smem);
   PrefillSmem& sm = sm2.t;
   pdl_begin();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
   const int qb = static_cast<int>(gridDim.x - 1 - blockIdx.x);
-  const int hkv = blockIdx.y, head = hkv * kPfWarps + warp;
+  const int head = blockIdx.y, hkv = head / kPfWarps, mt = warp & 1, nb0 = (warp >> 1) * 8;  // first 8-dim block
   const int r0 = qb * kQRows2;
   const int nrows = min(kQRows2, p.rows - r0);
   const int kv_len = p.base_pos + r0 + nrows;
   const int ntiles = (kv_len + kTileP - 1) / kTileP;
   const size_t head_row0 = static_cast<size_t>(hkv) * p.stride;
-  int pos_row[2][2];  // [tile of 16 rows][row g / g + 8]
+  int pos_row[2];  // rows g and g + 8 of the tile
 #pragma unroll
-  for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-    for (int e = 0; e < 2; ++e) pos_row[mt][e] = p.base_pos + r0 + min(mt * 16 + g + 8 * e, nrows - 1);
+  for (int e = 0; e < 2; ++e) pos_row[e] = p.base_pos + r0 + min(mt * 16 + g + 8 * e, nrows - 1);
 
   const int crow = tid >> 1, chalf = tid & 1;
   auto gather = [&](int stage, int tile) {
@@ -332,25 +333,20 @@ __global__ void __launch_bounds__(kPfWarps * 32, 2) attn_prefill2_kernel(const P
   };
   gather(0, 0);
 
-  // this warp's 32 Q rows -> fp16 in shared memory (rows past the chunk repeat the last row)
-  for (int i = lane; i < kQRows2 * (kD / 8); i += 32) {
+  // the Q rows -> fp16 in shared memory (rows past the chunk repeat the last row); read behind the tile loop's barrier
+  for (int i = tid; i < kQRows2 * (kD / 8); i += kWarps2 * 32) {
     const int row = i >> 4, piece = i & 15;
     const uint4 w = __ldg(reinterpret_cast<const uint4*>(p.q + (static_cast<size_t>(r0 + min(row, nrows - 1)) * p.Hq + head) * kD) + piece);
     uint4 h;
     h.x = pf_pack(bf16_lo(w.x), bf16_hi(w.x)), h.y = pf_pack(bf16_lo(w.y), bf16_hi(w.y));
     h.z = pf_pack(bf16_lo(w.z), bf16_hi(w.z)), h.w = pf_pack(bf16_lo(w.w), bf16_hi(w.w));
-    *reinterpret_cast<uint4*>(&sm2.qh[warp][row][piece * 8]) = h;
+    *reinterpret_cast<uint4*>(&sm2.qh[row][piece * 8]) = h;
   }
-  __syncwarp();
 
-  float o[2][16][4];
+  float o[8][4];  // dims 8 (nb0 + nb) ..
 #pragma unroll
-  for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-    for (int nb = 0; nb < 16; ++nb) o[mt][nb][0] = o[mt][nb][1] = o[mt][nb][2] = o[mt][nb][3] = 0.0f;
-  float m_run[2][2], l_run[2][2];
-#pragma unroll
-  for (int mt = 0; mt < 2; ++mt) m_run[mt][0] = m_run[mt][1] = -INFINITY, l_run[mt][0] = l_run[mt][1] = 0.0f;
+  for (int nb = 0; nb < 8; ++nb) o[nb][0] = o[nb][1] = o[nb][2] = o[nb][3] = 0.0f;
+  float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.0f, 0.0f};
 
   for (int tile = 0; tile < ntiles; ++tile) {
     const int stage = tile & 1;
@@ -358,8 +354,8 @@ __global__ void __launch_bounds__(kPfWarps * 32, 2) attn_prefill2_kernel(const P
     __syncthreads();
     if (tile + 1 < ntiles) gather(stage ^ 1, tile + 1);
 #pragma unroll
-    for (int it = 0; it < kTileP * 16 / (kPfWarps * 32); ++it) {
-      const int item = it * (kPfWarps * 32) + tid, row = item >> 4, piece = item & 15;
+    for (int it = 0; it < kTileP * 16 / (kWarps2 * 32); ++it) {
+      const int item = it * (kWarps2 * 32) + tid, row = item >> 4, piece = item & 15;
       const uint2 rk = *reinterpret_cast<const uint2*>(&sm.raw_k[stage][row][piece * 8]);
       const uint2 rv = *reinterpret_cast<const uint2*>(&sm.raw_v[stage][row][piece * 8]);
       const __half2 vs2 = __float2half2_rn(sm.vs[stage][row]);
@@ -378,20 +374,16 @@ __global__ void __launch_bounds__(kPfWarps * 32, 2) attn_prefill2_kernel(const P
     for (int half = 0; half < 2; ++half) {  // 32 positions at a time
       const int c0 = tile * kTileP + half * 32;
       if (c0 >= kv_len) break;  // uniform over the CTA
-      // ---- S = Q K^T: two 16 x 32 tiles; a K fragment serves both
-      float s[2][4][4];
+      // ---- S = Q K^T: 16 x 32
+      float s[4][4];
 #pragma unroll
-      for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) s[mt][j][0] = s[mt][j][1] = s[mt][j][2] = s[mt][j][3] = 0.0f;
+      for (int j = 0; j < 4; ++j) s[j][0] = s[j][1] = s[j][2] = s[j][3] = 0.0f;
 #pragma unroll
       for (int kk = 0; kk < 8; kk += 2) {
-        uint32_t qa[2][2][4];  // [row tile][k-step kk, kk + 1]
+        uint32_t qa[2][4];  // k-steps kk, kk + 1
 #pragma unroll
-        for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-          for (int u = 0; u < 2; ++u)
-            pf_ldmatrix_x4(qa[mt][u], &sm2.qh[warp][mt * 16 + (lane & 7) + ((lane >> 3) & 1) * 8][(kk + u) * 16 + (lane >> 4) * 8]);
+        for (int u = 0; u < 2; ++u)
+          pf_ldmatrix_x4(qa[u], &sm2.qh[mt * 16 + (lane & 7) + ((lane >> 3) & 1) * 8][(kk + u) * 16 + (lane >> 4) * 8]);
 #pragma unroll
         uint32_t b[4][4];
 #pragma unroll
@@ -399,88 +391,81 @@ __global__ void __launch_bounds__(kPfWarps * 32, 2) attn_prefill2_kernel(const P
 #pragma unroll
         for (int u = 0; u < 2; ++u)  // no two consecutive MMAs share an accumulator
 #pragma unroll
-          for (int j = 0; j < 4; ++j)
-#pragma unroll
-            for (int mt = 0; mt < 2; ++mt) pf_mma(s[mt][j], qa[mt][u], b[j][2 * u], b[j][2 * u + 1]);
+          for (int j = 0; j < 4; ++j) pf_mma(s[j], qa[u], b[j][2 * u], b[j][2 * u + 1]);
       }
       // ---- scale, mask, online softmax; P fragments
       const bool diag = c0 + 31 > p.base_pos + r0;
-      uint32_t pa[2][2][4];
-#pragma unroll
-      for (int mt = 0; mt < 2; ++mt) {
+      uint32_t pa[2][4];
+      {
         float mx[2] = {-INFINITY, -INFINITY};
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           const float2 f = *reinterpret_cast<const float2*>(&sm.ks[stage][half * 32 + j * 8 + 2 * t]);
-          s[mt][j][0] *= f.x, s[mt][j][1] *= f.y, s[mt][j][2] *= f.x, s[mt][j][3] *= f.y;
+          s[j][0] *= f.x, s[j][1] *= f.y, s[j][2] *= f.x, s[j][3] *= f.y;
           if (diag) {
             const int col = c0 + j * 8 + 2 * t;
-            if (col > pos_row[mt][0]) s[mt][j][0] = -INFINITY;
-            if (col + 1 > pos_row[mt][0]) s[mt][j][1] = -INFINITY;
-            if (col > pos_row[mt][1]) s[mt][j][2] = -INFINITY;
-            if (col + 1 > pos_row[mt][1]) s[mt][j][3] = -INFINITY;
+            if (col > pos_row[0]) s[j][0] = -INFINITY;
+            if (col + 1 > pos_row[0]) s[j][1] = -INFINITY;
+            if (col > pos_row[1]) s[j][2] = -INFINITY;
+            if (col + 1 > pos_row[1]) s[j][3] = -INFINITY;
           }
-          mx[0] = fmaxf(mx[0], fmaxf(s[mt][j][0], s[mt][j][1]));
-          mx[1] = fmaxf(mx[1], fmaxf(s[mt][j][2], s[mt][j][3]));
+          mx[0] = fmaxf(mx[0], fmaxf(s[j][0], s[j][1]));
+          mx[1] = fmaxf(mx[1], fmaxf(s[j][2], s[j][3]));
         }
         float corr[2], base[2], rsum[2] = {0.0f, 0.0f};
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
           mx[e] = fmaxf(mx[e], __shfl_xor_sync(0xffffffffu, mx[e], 1));
           mx[e] = fmaxf(mx[e], __shfl_xor_sync(0xffffffffu, mx[e], 2));
-          const float m_new = fmaxf(m_run[mt][e], mx[e]);
-          corr[e] = m_new == -INFINITY ? 1.0f : pf_ex2(m_run[mt][e] - m_new);
+          const float m_new = fmaxf(m_run[e], mx[e]);
+          corr[e] = m_new == -INFINITY ? 1.0f : pf_ex2(m_run[e] - m_new);
           base[e] = m_new == -INFINITY ? 0.0f : m_new;
-          m_run[mt][e] = m_new;
+          m_run[e] = m_new;
         }
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          const float p0 = pf_ex2(s[mt][j][0] - base[0]), p1 = pf_ex2(s[mt][j][1] - base[0]);
-          const float p2 = pf_ex2(s[mt][j][2] - base[1]), p3 = pf_ex2(s[mt][j][3] - base[1]);
+          const float p0 = pf_ex2(s[j][0] - base[0]), p1 = pf_ex2(s[j][1] - base[0]);
+          const float p2 = pf_ex2(s[j][2] - base[1]), p3 = pf_ex2(s[j][3] - base[1]);
           rsum[0] += p0 + p1, rsum[1] += p2 + p3;
-          pa[mt][j >> 1][(j & 1) * 2] = pf_pack(p0, p1);
-          pa[mt][j >> 1][(j & 1) * 2 + 1] = pf_pack(p2, p3);
+          pa[j >> 1][(j & 1) * 2] = pf_pack(p0, p1);
+          pa[j >> 1][(j & 1) * 2 + 1] = pf_pack(p2, p3);
         }
-        l_run[mt][0] = l_run[mt][0] * corr[0] + rsum[0], l_run[mt][1] = l_run[mt][1] * corr[1] + rsum[1];
+        l_run[0] = l_run[0] * corr[0] + rsum[0], l_run[1] = l_run[1] * corr[1] + rsum[1];
         if (__any_sync(0xffffffffu, corr[0] != 1.0f || corr[1] != 1.0f)) {
 #pragma unroll
-          for (int nb = 0; nb < 16; ++nb)
-            o[mt][nb][0] *= corr[0], o[mt][nb][1] *= corr[0], o[mt][nb][2] *= corr[1], o[mt][nb][3] *= corr[1];
+          for (int nb = 0; nb < 8; ++nb)
+            o[nb][0] *= corr[0], o[nb][1] *= corr[0], o[nb][2] *= corr[1], o[nb][3] *= corr[1];
         }
       }
-      // ---- O += P V: a V fragment serves both row tiles
+      // ---- O += P V
 #pragma unroll
       for (int kk = 0; kk < 2; ++kk) {
 #pragma unroll
-        for (int nb = 0; nb < 16; nb += 2) {
+        for (int nb = 0; nb < 8; nb += 2) {
           uint32_t b[4];
-          pf_ldmatrix_x4_trans(b, &sm.vh[half * 32 + kk * 16 + (lane & 7) + ((lane >> 3) & 1) * 8][nb * 8 + (lane >> 4) * 8]);
-#pragma unroll
-          for (int mt = 0; mt < 2; ++mt) {
-            pf_mma(o[mt][nb], pa[mt][kk], b[0], b[1]);
-            pf_mma(o[mt][nb + 1], pa[mt][kk], b[2], b[3]);
-          }
+          pf_ldmatrix_x4_trans(b, &sm.vh[half * 32 + kk * 16 + (lane & 7) + ((lane >> 3) & 1) * 8][(nb0 + nb) * 8 + (lane >> 4) * 8]);
+          pf_mma(o[nb], pa[kk], b[0], b[1]);
+          pf_mma(o[nb + 1], pa[kk], b[2], b[3]);
         }
       }
     }
   }
 
-#pragma unroll
-  for (int mt = 0; mt < 2; ++mt) {
+  {
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
-      l_run[mt][e] += __shfl_xor_sync(0xffffffffu, l_run[mt][e], 1);
-      l_run[mt][e] += __shfl_xor_sync(0xffffffffu, l_run[mt][e], 2);
+      l_run[e] += __shfl_xor_sync(0xffffffffu, l_run[e], 1);
+      l_run[e] += __shfl_xor_sync(0xffffffffu, l_run[e], 2);
     }
-    const float inv_a = l_run[mt][0] > 0.0f ? 1.0f / l_run[mt][0] : 0.0f;
-    const float inv_b = l_run[mt][1] > 0.0f ? 1.0f / l_run[mt][1] : 0.0f;
+    const float inv_a = l_run[0] > 0.0f ? 1.0f / l_run[0] : 0.0f;
+    const float inv_b = l_run[1] > 0.0f ? 1.0f / l_run[1] : 0.0f;
     const int ra = mt * 16 + g, rb = ra + 8;
-    uint16_t* out_a = p.out + (static_cast<size_t>(r0 + ra) * p.Hq + head) * kD + 2 * t;
-    uint16_t* out_b = p.out + (static_cast<size_t>(r0 + rb) * p.Hq + head) * kD + 2 * t;
+    uint16_t* out_a = p.out + (static_cast<size_t>(r0 + ra) * p.Hq + head) * kD + nb0 * 8 + 2 * t;
+    uint16_t* out_b = p.out + (static_cast<size_t>(r0 + rb) * p.Hq + head) * kD + nb0 * 8 + 2 * t;
 #pragma unroll
-    for (int nb = 0; nb < 16; ++nb) {
-      if (ra < nrows) *reinterpret_cast<uint32_t*>(out_a + nb * 8) = pack_bf16x2(o[mt][nb][0] * inv_a, o[mt][nb][1] * inv_a);
-      if (rb < nrows) *reinterpret_cast<uint32_t*>(out_b + nb * 8) = pack_bf16x2(o[mt][nb][2] * inv_b, o[mt][nb][3] * inv_b);
+    for (int nb = 0; nb < 8; ++nb) {
+      if (ra < nrows) *reinterpret_cast<uint32_t*>(out_a + nb * 8) = pack_bf16x2(o[nb][0] * inv_a, o[nb][1] * inv_a);
+      if (rb < nrows) *reinterpret_cast<uint32_t*>(out_b + nb * 8) = pack_bf16x2(o[nb][2] * inv_b, o[nb][3] * inv_b);
     }
   }
 }
@@ -519,8 +504,8 @@ int attn_prefill_flash(const char* fn, const uint16_t* d_q, float scale, int Hq,
   p.scale_log2 = scale * 1.4426950408889634f;
   const char* v = std::getenv("G4_PREFILL_ROWS32");  // 0: 16 query positions per CTA
   if (!(v != nullptr && v[0] == '0')) {
-    const dim3 grid(static_cast<unsigned>((rows + kQRows2 - 1) / kQRows2), static_cast<unsigned>(Hk));
-    G4_LAUNCH_PDL(fn, attn_prefill2_kernel, grid, dim3(kPfWarps * 32), sizeof(PrefillSmem2), current_stream(), p);
+    const dim3 grid(static_cast<unsigned>((rows + kQRows2 - 1) / kQRows2), static_cast<unsigned>(Hq));
+    G4_LAUNCH_PDL(fn, attn_prefill2_kernel, grid, dim3(kWarps2 * 32), sizeof(PrefillSmem2), current_stream(), p);
     return 0;
   }
   const dim3 grid(static_cast<unsigned>((rows + kQRows - 1) / kQRows), static_cast<unsigned>(Hk));

@@ -184,3 +184,17 @@ def test_output_that_is_not_16_byte_aligned(K):
     assert K.prefill_attention_int8(dev(q), SCALE, Hq, Hk, D, 0, stride, out, *[dev(x) for x in pl], pt=None) == 0
     got = out.cpu().numpy().view(np.uint16)
     assert close(f32_of(got), f32_of(want), 0.01) and int(buf[:2].abs().sum()) == 0 and int(buf[-6:].abs().sum()) == 0
+
+
+@pytest.mark.parametrize("rows,base", [(32, 0), (33, 1000), (48, 63), (63, 1985)])
+def test_chunks_below_the_tensor_core_form(K, rows, base):
+    """32 - 63 rows (one query head, two row tiles and two halves of the dims per CTA): ragged row tiles, rows whose
+    mask starts in any half tile; every row against float64."""
+    stride = 2048
+    pl = pool(rows, stride)
+    rng = np.random.default_rng(rows + base)
+    table = rng.permutation(stride).astype(np.int32)
+    q = bf16_bits(2.0 * rng.standard_normal((rows, Hq * D)))
+    got = run(K, q, pl, base, stride, table)
+    exact = f64_rows(q, pl, [table] * rows, (base + np.arange(rows)).astype(np.int32))
+    assert close(f32_of(got).reshape(rows, Hq, D), exact, 0.01)
