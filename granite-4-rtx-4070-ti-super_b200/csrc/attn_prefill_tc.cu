@@ -21,7 +21,9 @@
 // cache range of a block is then split over the CTAs of a thread-block cluster (plan_splits): each walks
 // its share of the tiles with its own softmax state, and the partial O rows meet in distributed shared
 // memory as a reduce-scatter - rank o finishes a contiguous part of the 256 rows - so that no workspace
-// in global memory and no second launch are needed. PLACEHOLDER_MEASURED
+// in global memory and no second launch are needed. 64 rows after 30000 positions 591 us in one
+// CTA per block, 79 in ten; 128 rows after 4000 93 and 33 (six); 500 after 16000 385 and 205 (two); 700 after
+// 30000 707 and 469 (three).
 //
 // Roles by warp (14 warps; every hand-over is an mbarrier, every wait on one is bounded):
 //   warp 0      producer: looks the tile's 64 positions up in the page table and fetches their raw
@@ -695,7 +697,8 @@ static int resident_ctas(int splits) {
 // its tiles (Q rows, first pages, the last P V: kFixed; the look at tile 0 and the exchange: kExchange). Fewer
 // CTAs win a tie. From four rounds on the rounds are full enough and nothing is split. Large clusters lose by
 // themselves: few of them fit between the chip's SM clusters. G4_PREFILL_SPLITS forces a count (tests,
-// measurements). PLACEHOLDER_PLAN
+// measurements). Measured, 128 rows after 4000: 1 CTA per block 93 us, 4 40, 6 33 (the plan), 8 54;
+// 256 rows after 16000: 1 327, 3 127, 4 100 (the plan), 6 141; 1999 rows after 30000: 1 1253 (the plan), 3 1314.
 static int plan_splits(int rows, int base_pos, int Hk) {
   constexpr double kFixed = 3.0, kExchange = 3.0;
   if (const char* v = std::getenv("G4_PREFILL_SPLITS"); v != nullptr && std::atoi(v) > 0) {
