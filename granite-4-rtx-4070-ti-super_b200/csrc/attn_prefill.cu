@@ -384,7 +384,6 @@ __global__ void __launch_bounds__(kWarps2 * 32, 2) attn_prefill2_kernel(const Pr
 #pragma unroll
         for (int u = 0; u < 2; ++u)
           pf_ldmatrix_x4(qa[u], &sm2.qh[mt * 16 + (lane & 7) + ((lane >> 3) & 1) * 8][(kk + u) * 16 + (lane >> 4) * 8]);
-#pragma unroll
         uint32_t b[4][4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) pf_ldmatrix_x4(b[j], &sm.kh[half * 32 + j * 8 + (lane & 7)][kk * 16 + (lane >> 3) * 8]);
