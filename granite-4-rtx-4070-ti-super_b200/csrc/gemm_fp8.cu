@@ -531,14 +531,14 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
   tc_fence_after();
   const uint32_t tmem_base = ring->tmem_base;
 
-  // Programmatic dependent launch. Everything above touches no global memory. The weights are
-  // constants of the model, not products of the kernel before this one on the stream, so the W
-  // loader does not wait for that kernel; whatever reads activations, residuals, scales or the
-  // workspace, and everything that writes, comes after the wait. The decode-size forms (p.early) also
-  // let the kernel after them start as soon as CTAs of this one retire: with a few microseconds of
-  // work per launch, the ramps of consecutive GEMMs are most of the time otherwise.
+  // Programmatic dependent launch. Everything above touches no global memory. At more than 128 rows every
+  // warp waits for the kernel ahead, the W loaders too: W may then be written by any operation before this
+  // call, and fetching it early would hide about a microsecond. The decode-size forms (p.early) take W for a
+  // constant of the model and let its loaders run ahead of that wait (granite4_b200.h states what this asks
+  // of the caller), and let the kernel after them start as soon as CTAs of this one retire: with a few
+  // microseconds of work per launch, the ramps of consecutive GEMMs are most of the time otherwise.
   if (p.early) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  if (warp != 0 && warp != 7) asm volatile("griddepcontrol.wait;" ::: "memory");
+  if (!p.early || (warp != 0 && warp != 7)) asm volatile("griddepcontrol.wait;" ::: "memory");
 
   const int bn = kPair ? p.bn : kBN;                  // accumulator columns of a tile
   const int tile_cols = p.swiglu_i ? bn / 2 : bn;     // output columns of a tile

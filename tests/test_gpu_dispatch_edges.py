@@ -132,3 +132,31 @@ def test_fused_swiglu_of_few_rows_equals_gemm_then_swiglu(K, M, inter, Kd):
     want, c8, sa = torch.empty_like(out), torch.empty(M, inter, dtype=torch.uint8, device=DEV), torch.zeros(2, device=DEV)
     assert K.swiglu_fp8(both[:, :inter].contiguous(), both[:, inter:].contiguous(), want, c8, sa) == 0
     assert torch.equal(out, want) and slot[1].item() == sa[1].item()
+
+
+@pytest.mark.parametrize("M,pair", [(129, True), (256, True), (256, False)])
+def test_weights_written_on_the_stream_just_before_the_gemm(K, monkeypatch, M, pair):
+    """At more than 128 rows W may come from any operation ahead of the call: it is rewritten for every call, once
+    with the quantisation of A between (small tensors, whose launches overlap), once as the operation just before.
+    The values are codes of themselves (amax 448, scale 1), so each product is a sum of whole numbers."""
+    if not pair:
+        monkeypatch.setenv("G4_GEMM_PAIR", "0")
+    n, kd, rounds = 256, 256, 40
+    g = torch.Generator(device=DEV).manual_seed(M)
+
+    def whole(r):
+        x = torch.randint(-2, 3, (rounds, r, kd), generator=g, device=DEV).to(torch.bfloat16)
+        x[:, 0, 0] = 448.0
+        return x
+    a, w = whole(M), whole(n)
+    a8, w8 = (torch.empty(r, kd, dtype=torch.uint8, device=DEV) for r in (M, n))
+    sa, sw = torch.zeros(2, device=DEV), torch.zeros(2, device=DEV)
+    out = torch.zeros(2, rounds, M, n, device=DEV)
+    for last_is_w in (0, 1):
+        for i in range(rounds):
+            ops = [(w[i], w8, sw), (a[i], a8, sa)]
+            for x, c, s in (reversed(ops) if last_is_w else ops):
+                assert K.fp8_quant(x, c, s) == 0
+            assert K.gemm_fp8(a8, w8, out[last_is_w, i], a_scale=sa) == 0
+    want = torch.matmul(a.double(), w.double().transpose(1, 2)).float()
+    assert torch.equal(out[0], want) and torch.equal(out[1], want)
