@@ -297,7 +297,9 @@ def gemm_fp8(a_fp8, w_fp8, out, a_scale=None, w_scales=(1.0,), segs=(), residual
     same pitch as out (GemmOut::kResidual, engine/src/prefill_gemm.h:12-16). workspace: uint8 CUDA
     tensor from gemm_fp8_workspace (zeroed once; reusable call after call). swiglu_scale_amax: float32[2];
     when given, w_fp8 is gate rows then up rows and out [M][N / 2] gets bf16(silu(gate) * up), its
-    max |.| going to swiglu_scale_amax[1] (GRANITE4_GEMM_OUT_SWIGLU)."""
+    max |.| going to swiglu_scale_amax[1] (GRANITE4_GEMM_OUT_SWIGLU).
+    With at most 128 rows w_fp8 must not be a product of the chain of this library's calls that leads up to
+    this one: its blocks are fetched while those calls still run (granite4_b200.h)."""
     return _n.gemm_fp8(a_fp8, w_fp8, out, a_scale, w_scales, segs, residual, resid_scale, workspace,
                        swiglu_scale_amax)
 

@@ -681,9 +681,15 @@ int granite4_prefill_attention_int8(const uint16_t* d_q_rot, float scale, int Hq
  * reported a non-zero word (a bounded wait ran out and the kernel left early),
  * or after a failed launch, zero the buffer again before reusing it, or later
  * calls sum stale partials without reporting anything. NULL or a smaller
- * buffer: no split. d_w must not be written by the operation just before this call on
- * the stream: with at most 128 rows the kernel starts fetching weights while
- * that operation drains (weights are constants of a loaded model). Returns 0,
+ * buffer: no split.
+ * With at most 128 rows d_w has to be complete when the calls begin that lead up to
+ * this one: the kernel starts fetching weights while calls of this library ahead of
+ * it on the stream still run, and with small launches that is more than the last one
+ * (weights are constants of a loaded model). A W that is written on the same stream
+ * is complete once an operation of another kind stands between its writer and this
+ * call: a copy, a memset, a wait for an event, or a kernel launched without
+ * programmatic serialisation. With more than 128 rows the kernel waits for everything
+ * ahead of it, and W may come from any operation before the call. Returns 0,
  * or -1 on bad arguments or a launch error. */
 enum {
   GRANITE4_GEMM_OUT_BF16 = 0,
