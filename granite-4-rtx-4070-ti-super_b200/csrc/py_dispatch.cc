@@ -74,6 +74,16 @@ const at::Tensor& tensor(PyObject* o) {
   return THPVariable_Unpack(o);
 }
 
+// A tensor whose two dimensions are an entry point's rows and columns.
+const at::Tensor& matrix(PyObject* o) {
+  const at::Tensor& t = tensor(o);
+  if (t.dim() != 2) {
+    PyErr_Format(PyExc_ValueError, "expected a matrix, got a tensor of %d dimensions", static_cast<int>(t.dim()));
+    throw PyErrorSet{};
+  }
+  return t;
+}
+
 // Device pointer of a contiguous CUDA tensor of one of the given types (None passes through as NULL).
 template <typename T = void>
 T* ptr(PyObject* o, Types types = kAny) {
@@ -191,7 +201,7 @@ OP(rmsnorm, 7) {  // x, w, eps, rows, cols, out, batched
 }
 
 OP(add_rmsnorm_fp8, 10) {  // y, res, w, eps, resid_mult, h_out, n_bf16, n_fp8, scale_amax, rstd
-  const at::Tensor& y = tensor(a[0]);
+  const at::Tensor& y = matrix(a[0]);
   enter(y);
   const int rows = static_cast<int>(y.size(0)), cols = static_cast<int>(y.size(1));
   const int yf = y.scalar_type() == at::kFloat, rf = a[1] != Py_None && tensor(a[1]).scalar_type() == at::kFloat;
@@ -208,7 +218,7 @@ OP(add_rmsnorm_fp8, 10) {  // y, res, w, eps, resid_mult, h_out, n_bf16, n_fp8, 
 }
 
 OP(add_rmsnorm_fp8_noalloc, 8) {  // y, res, w, eps, resid_mult, h_out, n_fp8, scale_amax
-  const at::Tensor& y = tensor(a[0]);
+  const at::Tensor& y = matrix(a[0]);
   enter(y);
   const int rows = static_cast<int>(y.size(0)), cols = static_cast<int>(y.size(1));
   const int yf = y.scalar_type() == at::kFloat, rf = a[1] != Py_None && tensor(a[1]).scalar_type() == at::kFloat;
@@ -404,7 +414,7 @@ OP(rope_kv_int8_paged, 16) {  // qkv, cos, sin, pos_rows, kv_rows, Hq, Hk, d, st
 
 // ---- decode-step glue -----------------------------------------------------------------------------
 OP(argmax_rows, 4) {  // logits, out, d_pos, vocab_map
-  const at::Tensor& t = tensor(a[0]);
+  const at::Tensor& t = matrix(a[0]);
   enter(t);
   const auto* x = ptr<const uint16_t>(a[0], kBf16);
   const int rows = static_cast<int>(t.size(0)), V = static_cast<int>(t.size(1));
@@ -415,7 +425,7 @@ OP(argmax_rows, 4) {  // logits, out, d_pos, vocab_map
 }
 
 OP(argmax_advance, 3) {  // logits, d_rows, ids_out
-  const at::Tensor& t = tensor(a[0]);
+  const at::Tensor& t = matrix(a[0]);
   enter(t);
   const auto* x = ptr<const uint16_t>(a[0], kBf16);
   const int rows = static_cast<int>(t.size(0)), V = static_cast<int>(t.size(1));
@@ -593,7 +603,7 @@ OP(prefill_silu_mul, 4) {  // gu, I, rows, act
 }
 
 OP(swiglu_fp8, 6) {  // gate, up, act_bf16, act_fp8, scale_amax, ld
-  const at::Tensor &g = tensor(a[0]), &u = tensor(a[1]);
+  const at::Tensor &g = matrix(a[0]), &u = tensor(a[1]);
   enter(g);
   const int rows = static_cast<int>(g.size(0)), I = static_cast<int>(g.size(1));
   const long long ld = a[5] == Py_None ? g.stride(0) : whole(a[5]);

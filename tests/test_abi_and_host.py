@@ -142,6 +142,22 @@ def test_kernels_refuse_cpu_tensors(g4):
         kernels._p(x, torch.bfloat16)
 
 
+@pytest.mark.parametrize("shape", [(4096,), (2, 8, 4096)])
+def test_kernels_refuse_what_is_no_matrix(g4, shape):
+    """Where an entry point takes its rows and columns from the tensor, one or three dimensions are an error
+    (told before anything else about the tensor, so it can be tested without a GPU)."""
+    import torch
+    from granite4_b200 import kernels
+    x, w = torch.zeros(shape, dtype=torch.bfloat16), torch.zeros(4096, dtype=torch.bfloat16)
+    u8 = torch.zeros(shape, dtype=torch.uint8)
+    for call in (lambda: kernels.add_rmsnorm_fp8(x, None, w, 1e-5, 1.0, n_bf16=x),
+                 lambda: kernels.add_rmsnorm_fp8_noalloc(x, None, w, 1e-5, 1.0, x, u8, w),
+                 lambda: kernels.argmax_rows(x, w), lambda: kernels.argmax_advance(x, u8),
+                 lambda: kernels.swiglu_fp8(x, x, act_bf16=x)):
+        with pytest.raises(ValueError, match="expected a matrix"):
+            call()
+
+
 def test_row_table_follows_the_pool_rule(g4):
     from granite4_b200 import paging
     # engine/src/kv_pool.cc:285-298: out[p] = page_id * B + p % B
