@@ -530,17 +530,34 @@ OP(prefill_attention_int8, 14) {  // q_rot, scale, Hq, Hk, d, base_pos, stride, 
 }
 
 // ---- FP8 GEMM -----------------------------------------------------------------------------------------
-// The idx-th number of a sequence of n >= 1 (its last one past the end).
-double item_or_last(PyObject* seq, Py_ssize_t n, Py_ssize_t idx) {
-  PyObject* v = PySequence_GetItem(seq, idx < n ? idx : n - 1);
-  if (v == nullptr) throw PyErrorSet{};
-  const double d = PyFloat_AsDouble(v);
-  Py_DECREF(v);
-  if (d == -1.0 && PyErr_Occurred()) throw PyErrorSet{};
-  return d;
-}
+// The items of any iterable, as a tuple that this object owns.
+struct Items {
+  PyObject* seq;
+  explicit Items(PyObject* o) : seq(PySequence_Tuple(o)) {
+    if (seq == nullptr) throw PyErrorSet{};
+  }
+  ~Items() { Py_DECREF(seq); }
+  Items(const Items&) = delete;
+  Items& operator=(const Items&) = delete;
+  Py_ssize_t size() const { return PyTuple_GET_SIZE(seq); }
+  PyObject* item(Py_ssize_t i) const { return PyTuple_GET_ITEM(seq, i); }
+  PyObject* item_or_last(Py_ssize_t i) const { return item(i < size() ? i : size() - 1); }
+};
 
 OP(gemm_fp8, 10) {  // a, w, out, a_scale, w_scales, segs, residual, resid_scale, workspace, swiglu_scale_amax
+  granite4_gemm_fp8_epilogue ep{};
+  {
+    const Items ws(a[4]), sg(a[5]);
+    if (ws.size() < 1 || ws.size() > 3 || sg.size() > 2) {
+      PyErr_SetString(PyExc_ValueError, "one to three weight scales, at most two segment ends");
+      return nullptr;
+    }
+    ep.w_scale0 = real(ws.item_or_last(0));
+    ep.w_scale1 = real(ws.item_or_last(1));
+    ep.w_scale2 = real(ws.item_or_last(2));
+    ep.seg1 = sg.size() > 0 ? num(sg.item(0)) : INT32_MAX;
+    ep.seg2 = sg.size() > 1 ? num(sg.item(1)) : INT32_MAX;
+  }
   const at::Tensor& A = tensor(a[0]);
   enter(A);
   const at::Tensor &W = tensor(a[1]), &out = tensor(a[2]);
@@ -549,19 +566,7 @@ OP(gemm_fp8, 10) {  // a, w, out, a_scale, w_scales, segs, residual, resid_scale
     PyErr_SetString(PyExc_ValueError, "a_fp8 / w_fp8 must be uint8 code matrices with unit column stride");
     return nullptr;
   }
-  granite4_gemm_fp8_epilogue ep{};
   ep.d_a_scale = ptr<const float>(a[3], kF32);
-  const Py_ssize_t nw = PySequence_Size(a[4]), ns = PySequence_Size(a[5]);
-  if (nw < 0 || ns < 0) return nullptr;
-  if (nw < 1 || nw > 3 || ns > 2) {
-    PyErr_SetString(PyExc_ValueError, "one to three weight scales, at most two segment ends");
-    return nullptr;
-  }
-  ep.w_scale0 = static_cast<float>(item_or_last(a[4], nw, 0));
-  ep.w_scale1 = static_cast<float>(item_or_last(a[4], nw, 1));
-  ep.w_scale2 = static_cast<float>(item_or_last(a[4], nw, 2));
-  ep.seg1 = ns > 0 ? static_cast<int>(item_or_last(a[5], ns, 0)) : INT32_MAX;
-  ep.seg2 = ns > 1 ? static_cast<int>(item_or_last(a[5], ns, 1)) : INT32_MAX;
   ep.resid_scale = real(a[7]);
   ep.ldc = static_cast<int>(out.stride(0));
   int kind = GRANITE4_GEMM_OUT_BF16;

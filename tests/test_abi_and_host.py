@@ -158,6 +158,21 @@ def test_kernels_refuse_what_is_no_matrix(g4, shape):
             call()
 
 
+def test_gemm_scales_and_segments_are_taken_as_before(g4):
+    """Any iterable of numbers gives the weight scales; a segment end is a whole number. (Read before the tensors,
+    whose place on the CPU is what ends the calls that are otherwise right.)"""
+    import torch
+    from granite4_b200 import kernels
+    u8, out = torch.zeros(8, 128, dtype=torch.uint8), torch.zeros(8, 8, dtype=torch.bfloat16)
+    for scales in ((1.0,), [1, 2.0], np.ones(3, np.float32), (s for s in (1.0, 2.0)), {1.0: None}):
+        with pytest.raises(ValueError, match="CUDA tensor"):
+            kernels.gemm_fp8(u8, u8, out, w_scales=scales, segs=iter([4]))
+    for kw, error in (({"w_scales": ()}, ValueError), ({"w_scales": (1.0,) * 4}, ValueError), ({"w_scales": 1.0}, TypeError),
+                      ({"w_scales": ("x",)}, TypeError), ({"segs": (1, 2, 3)}, ValueError), ({"segs": (4.5,)}, TypeError)):
+        with pytest.raises(error, match="^(?!.*CUDA tensor)"):
+            kernels.gemm_fp8(u8, u8, out, **kw)
+
+
 def test_row_table_follows_the_pool_rule(g4):
     from granite4_b200 import paging
     # engine/src/kv_pool.cc:285-298: out[p] = page_id * B + p % B
