@@ -247,6 +247,7 @@ def attn_decode_int8_paged(q, cache_k, cache_v, k_scale, v_scale, row_pos, Hq, H
     (``table.data_ptr()`` values), pt: one int32 table for every row; scratch: uint8 CUDA tensor of
     at least attn_decode_scratch_bytes(...) bytes (allocated here when not given)."""
     if scratch is None:
+        _n.enter_device_of(q)  # the size depends on the device
         need = capi.lib().granite4_attn_decode_scratch_bytes(q.shape[0], rows_per_group, Hk, max_len)
         if need > 0:
             scratch = torch.empty(need, dtype=torch.uint8, device=q.device)
@@ -261,6 +262,7 @@ def attn_split_int8(q, cache_k, cache_v, k_scale, v_scale, scale, Hq, Hk, d, str
     over the int8 pool. row_pt: int64 CUDA tensor of per-row table addresses; row_grp: int32 group
     words r0 | nr << 8; row_tbase int32 [rows], row_tail int32 [rows][8]."""
     if scratch is None:
+        _n.enter_device_of(q)  # the size depends on the device
         need = capi.lib().granite4_attn_split_scratch_bytes(Hq, q.shape[0], max_len if max_len > 0 else stride)
         scratch = torch.empty(max(need, 16), dtype=torch.uint8, device=q.device)
     return _n.attn_split_int8(q, cache_k, cache_v, k_scale, v_scale, scale, Hq, Hk, d, stride, out, kv_base, d_pos, pt,

@@ -173,6 +173,21 @@ def test_gemm_scales_and_segments_are_taken_as_before(g4):
             kernels.gemm_fp8(u8, u8, out, **kw)
 
 
+def test_attention_scratch_is_sized_for_the_device_of_the_queries(g4, monkeypatch):
+    """The size depends on the current device's SM count, so the queries' device is selected before it is asked for
+    (here: their place on the CPU is noticed first)."""
+    import torch
+    from granite4_b200 import capi, kernels
+    with pytest.raises(ValueError, match="CUDA tensor"):
+        kernels._n.enter_device_of(torch.zeros(1))  # binds the entry points
+    monkeypatch.setattr(capi, "lib", lambda: pytest.fail("asked for the size first"))
+    q, u = torch.zeros(1, 4096, dtype=torch.bfloat16), torch.zeros(8, dtype=torch.int8)
+    with pytest.raises(ValueError, match="CUDA tensor"):
+        kernels.attn_decode_int8_paged(q, u, u, q, q, u, 32, 8, 128, 16, 16, 1.0, q)
+    with pytest.raises(ValueError, match="CUDA tensor"):
+        kernels.attn_split_int8(q, u, u, q, q, 1.0, 32, 8, 128, 16, q)
+
+
 def test_row_table_follows_the_pool_rule(g4):
     from granite4_b200 import paging
     # engine/src/kv_pool.cc:285-298: out[p] = page_id * B + p % B
