@@ -333,13 +333,13 @@ __global__ void __launch_bounds__(kThreads, 1) attn_prefill_tc_kernel(const TcPa
     // The warp runs the loop together and one lane issues every MMA (elect_one): the descriptors stay in
     // uniform registers. With the loop under `if (lane == 0)` an MMA held the thread for ~45 ns, 24 of them
     // most of a tile's 1.85 us: a prefill chunk of 1999 rows after 30000 positions took 1675 us, 1400 now, 8192 rows from 0 906 and 760.
-    bool ok = wait_tc(&sm->q_ready, 0, sm, p.status);
+    bool ok = warp_agrees(wait_tc(&sm->q_ready, 0, sm, p.status));
     // (the address field has 14 bits; in a cluster the rank stands in the bits above and would run into the offset)
     const uint32_t q_lo = ((smem_u32(sm->q16[0]) >> 4) & 0x3fffu) | (1u << 16), k_lo = ((smem_u32(sm->k16[0]) >> 4) & 0x3fffu) | (1u << 16);
     const uint32_t v_lo = ((smem_u32(sm->v16[0]) >> 4) & 0x3fffu) | ((kKvTileBytes / 2 >> 4) << 16);  // 64-dim halves 8 KB apart
     auto issue_s = [&](int j) {
       const int b = j % kBufs, sb = j & 1;
-      if (!(ok = ok && wait_tc(&sm->kv_full[b], (j / kBufs) & 1, sm, p.status))) return;
+      if (!(ok = ok && warp_agrees(wait_tc(&sm->kv_full[b], (j / kBufs) & 1, sm, p.status)))) return;
       tc_fence_after();
       if (elect_one()) {
 #pragma unroll
@@ -359,7 +359,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_prefill_tc_kernel(const TcPa
       if (j + 1 < n_kv) issue_s(j + 1);
       const int b = j % kBufs, sb = j & 1;
       for (int t = 0; t < row_tiles && ok; ++t) {
-        if (!(ok = wait_tc(&sm->p_full[t][sb], (j >> 1) & 1, sm, p.status))) break;
+        if (!(ok = warp_agrees(wait_tc(&sm->p_full[t][sb], (j >> 1) & 1, sm, p.status)))) break;
         tc_fence_after();
         if (elect_one()) {
           if (j >= probe) {

@@ -82,6 +82,10 @@ __device__ __forceinline__ bool elect_one() {
       : "=r"(e));
   return e != 0u;
 }
+// The verdict of a bounded wait that every lane of a warp made for itself, as one verdict: true if all of them
+// saw the phase complete. When a wait runs out, lanes may disagree, and what follows such a wait in a role run
+// by a whole warp (elect.sync, tensor-memory loads, __syncwarp) has to be reached by all 32 or by none.
+__device__ __forceinline__ bool warp_agrees(bool ok) { return __all_sync(0xffffffffu, ok) != 0; }
 // Index of the warp in its CTA, as a value the compiler knows to be the same in every lane.
 __device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, int(threadIdx.x) >> 5, 0); }
 // 32 lanes x 32 consecutive 32-bit columns: thread t of the warp gets lane (base lane + t).

@@ -410,7 +410,7 @@ __device__ __forceinline__ uint32_t store_slabs(const GemmParams& p, const CUten
   for (int n = n0; n < n_end; n += width, ++st.count) {
     const uint32_t slab = st.base + (st.count & 1u) * kSlabBytes;
     if (resid) {
-      if (!wait_or_abort(st.res_full + (st.count & 1u), (st.count >> 1) & 1u, ring, p.status)) {
+      if (!warp_agrees(wait_or_abort(st.res_full + (st.count & 1u), (st.count >> 1) & 1u, ring, p.status))) {
         ok = false;
         break;
       }
@@ -598,11 +598,11 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
       for (int u = first; u < units && ok; u += step, ++local) {
         const int kb0 = (u % p.splits) * p.kb_per, kb1 = min(kblocks, kb0 + p.kb_per);
         const uint32_t acc = local & 1u, aph = (local >> 1) & 1u;
-        if (!(ok = wait_or_abort(&ring->acc_empty[acc], aph ^ 1u, ring, p.status))) break;
+        if (!(ok = warp_agrees(wait_or_abort(&ring->acc_empty[acc], aph ^ 1u, ring, p.status)))) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * kBN;
         for (int kb = kb0; kb < kb1; ++kb) {
-          if (!(ok = wait_or_abort(&ring->full[s], ph, ring, p.status))) break;
+          if (!(ok = warp_agrees(wait_or_abort(&ring->full[s], ph, ring, p.status)))) break;
           tc_fence_after();
           const uint32_t a_addr = tiles_addr + s * stage_bytes;
           const uint64_t a_desc = smem_desc_k128(a_addr), w_desc = smem_desc_k128(a_addr + kABytes);
@@ -636,7 +636,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
       const int n_end = min(p.swiglu_i ? p.swiglu_i : p.N, n0 + tile_cols);
       const bool live = row0 < p.M;  // uniform over the warp: a warp whose rows are all past M has nothing to do
       if (slabs && live && lane == 0 && p.out_kind == GRANITE4_GEMM_OUT_RESIDUAL) residual_ahead(&map_res, st, n0, n_end, row0);
-      ok = wait_or_abort(&ring->acc_full[acc], aph, ring, p.status);
+      ok = warp_agrees(wait_or_abort(&ring->acc_full[acc], aph, ring, p.status));
       if (p.splits > 1) ok = epilogue_all(ok);  // the split path below has barriers: leave it together or not at all
       if (!ok) break;
       tc_fence_after();
@@ -844,11 +844,11 @@ gemm_fp8_stream_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
     bool ok = true;
     for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x, ++local) {
       const uint32_t acc = local & 1u, aph = (local >> 1) & 1u;
-      if (!(ok = stream_wait(&ring->acc_empty[acc], aph ^ 1u, ring, p.status))) break;
+      if (!(ok = warp_agrees(stream_wait(&ring->acc_empty[acc], aph ^ 1u, ring, p.status)))) break;
       tc_fence_after();
       const uint32_t d_tmem = tmem_base + acc * kBN;
       for (int st = 0; st < stages_per_tile; ++st) {
-        if (!(ok = stream_wait(&ring->full[s], ph, ring, p.status))) break;
+        if (!(ok = warp_agrees(stream_wait(&ring->full[s], ph, ring, p.status)))) break;
         tc_fence_after();
         const uint32_t base = tiles_addr + s * stage_bytes;
         const int nblk = min(p.kc, kblocks - st * p.kc);
@@ -878,7 +878,7 @@ gemm_fp8_stream_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
     for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x, ++local) {
       const uint32_t acc = local & 1u, aph = (local >> 1) & 1u;
       const int n0 = t * w_rows, n_end = min(n_out, n0 + w_rows), row = q * 32 + lane;
-      if (!(ok = stream_wait(&ring->acc_full[acc], aph, ring, p.status))) break;
+      if (!(ok = warp_agrees(stream_wait(&ring->acc_full[acc], aph, ring, p.status)))) break;
       tc_fence_after();
       const uint32_t taddr = tmem_base + (uint32_t(q * 32) << 16) + acc * kBN;
       if (p.swiglu_i && q * 32 < p.M) {
@@ -1096,7 +1096,7 @@ gemm_fp8_decode_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
     uint32_t it = 0, s = 0, ph = 0;
     bool ok = true;
     for (int kb = kb0; kb < kb1 && ok; ++kb, ++it) {
-      if (!(ok = dec_wait(&ring->full[s], ph, ring, p.status))) break;
+      if (!(ok = warp_agrees(dec_wait(&ring->full[s], ph, ring, p.status)))) break;
       tc_fence_after();
       const uint32_t w_addr = tiles_addr + s * kDecStageBytes;
       const uint64_t w_desc = smem_desc_k128(w_addr), a_desc = smem_desc_k128(w_addr + kDecWBytes);
