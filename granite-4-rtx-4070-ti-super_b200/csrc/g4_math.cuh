@@ -205,12 +205,15 @@ __device__ __forceinline__ uint32_t fp8x2_quant(uint32_t w, F32x2 hi, F32x2 lo) 
   return fp8x2_encode(a, b);
 }
 
-// Eight packed bf16 values -> eight codes (element 0 in the low byte of .x).
-__device__ __forceinline__ uint2 fp8x8_quant(uint4 p, const Fp8Scale s) {
-  if (!s.plain) return fp8x8_quant_general(p, s.scale);  // uniform over the launch
+// Eight packed bf16 values -> eight codes (element 0 in the low byte of .x). The plain form is for kernels that
+// take the general one out of their main loop: the call in it costs them registers.
+__device__ __forceinline__ uint2 fp8x8_quant_plain(uint4 p, const Fp8Scale s) {
   const F32x2 hi = f32x2(s.hi, s.hi), lo = f32x2(s.lo, s.lo);
   return make_uint2(fp8x2_quant(p.x, hi, lo) | (fp8x2_quant(p.y, hi, lo) << 16),
                     fp8x2_quant(p.z, hi, lo) | (fp8x2_quant(p.w, hi, lo) << 16));
+}
+__device__ __forceinline__ uint2 fp8x8_quant(uint4 p, const Fp8Scale s) {
+  return s.plain ? fp8x8_quant_plain(p, s) : fp8x8_quant_general(p, s.scale);  // uniform over the launch
 }
 
 // ---- int8 KV rows (Q8_0) ----------------------------------------------------

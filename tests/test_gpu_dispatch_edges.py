@@ -112,6 +112,27 @@ def test_small_norm_quant_and_swiglu_equal_the_oracle(K, port, rows, cols):
     assert (c8.cpu().numpy() == cs).all() and sa[0].item() == ss and sa[1].item() == as_
 
 
+# powers of two on the weights: below, inside and above the range of the two-instruction quantiser
+@pytest.mark.parametrize("power", [-118, 0, 108])
+@pytest.mark.parametrize("rows,cols", [(17, 520), (20, 4096), (33, 4104)])
+def test_two_sweep_norm_under_unusual_scales_equals_the_oracle(K, port, rows, cols, power):
+    """More than 16 rows with rstd: the encode sweep reads the hidden state and 1/rms, and takes scales outside the
+    quantiser's plain range in a loop of its own."""
+    rng = np.random.default_rng(rows * 10007 + cols)
+
+    def bf(x):
+        return (np.ascontiguousarray(x, np.float32).view(np.uint32) >> 16).astype(np.uint16)
+    y, res = bf(rng.standard_normal((rows, cols))), bf(rng.standard_normal((rows, cols)))
+    w = bf(np.ldexp(rng.standard_normal(cols), power))
+    h, n = port.add_rmsnorm(y, res, w, 1e-5, 0.22)
+    codes, scale, amax = port.quant_fp8(n)
+    ho, c8 = torch.empty(rows, cols, dtype=torch.int16, device=DEV), torch.empty(rows, cols, dtype=torch.uint8, device=DEV)
+    sa, rstd = torch.full((2,), 9.0, device=DEV), torch.empty(rows, device=DEV)
+    assert K.add_rmsnorm_fp8(dev(y), dev(res), dev(w), 1e-5, 0.22, ho, None, c8, sa, rstd) == 0
+    assert (ho.cpu().numpy().view(np.uint16) == h).all()
+    assert (c8.cpu().numpy() == codes).all() and sa[0].item() == scale and sa[1].item() == amax
+
+
 @pytest.mark.parametrize("M,inter,Kd", [(1, 32, 128), (17, 96, 1552), (37, 1000, 512), (64, 12800, 256), (128, 200, 4096)])
 def test_fused_swiglu_of_few_rows_equals_gemm_then_swiglu(K, M, inter, Kd):
     """Gate and up rows as two parts of one tile: the f32 sums of these integer operands are exact, so the fused
