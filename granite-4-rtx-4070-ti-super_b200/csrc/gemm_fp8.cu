@@ -1423,8 +1423,10 @@ bool make_map3d(CUtensorMap* map, const void* base, int rows, int K, long long l
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+int a_rows_of(int M) { return (M + 15) / 16 * 16; }  // rows of A that the stream form fetches
+
 int launch_stream(const char* fn, const uint8_t* d_a, long long lda, const uint8_t* d_w, GemmParams p) {
-  p.a_rows = (p.M + 15) / 16 * 16;
+  p.a_rows = a_rows_of(p.M);
   const int n_out = p.swiglu_i ? p.swiglu_i : p.N;
   const StreamPlan pl = plan_stream(n_out, p.K, p.a_rows, sm_count(), p.swiglu_i != 0);
   const int w_rows = p.swiglu_i ? pl.bn / 2 : pl.bn;
@@ -1615,8 +1617,14 @@ extern "C" int granite4_kernel_gemm_fp8(int out_kind, const uint8_t* d_a, long l
   if (fused_swiglu) {
     p.swiglu_i = N / 2, p.amax_slot = ep->d_out_scale_amax;
     if (!amax_prezeroed()) G4_CUDA_TRY(fn, cudaMemsetAsync(p.amax_slot, 0, 2 * sizeof(float), current_stream()));
-    // no split of K under this epilogue; the tiled form's 128 output columns leave 48 SMs idle at I = 12800
-    if (M <= kBM) return stream_enabled() ? launch_stream(fn, d_a, lda, d_w, p) : launch<CfgWide>(fn, d_a, lda, d_w, p);
+    // No split of K under this epilogue. The stream form where a stage of its ring holds two k-blocks or more:
+    // with one, its single loader issues three copies per 128 bytes of K and sets the pace. K 4096, 64 and 128
+    // rows: I = 3072 16.8 and 18.6 us (tiled form 22.7 and 23.5), I = 6144 20.7 and, one block per stage, 32.0
+    // (24.8 and 24.8), I = 12800, one block, 33.1 and 34.0 (30.0 and 30.9).
+    if (M <= kBM) {
+      const bool stream = stream_enabled() && plan_stream(N / 2, K, a_rows_of(M), sm_count(), true).kc >= 2;
+      return stream ? launch_stream(fn, d_a, lda, d_w, p) : launch<CfgWide>(fn, d_a, lda, d_w, p);
+    }
   }
   if (M <= kDecRows && decode_form_enabled()) {
     const int rc = launch_decode(fn, d_a, lda, d_w, p);

@@ -133,7 +133,7 @@ def test_two_sweep_norm_under_unusual_scales_equals_the_oracle(K, port, rows, co
     assert (c8.cpu().numpy() == codes).all() and sa[0].item() == scale and sa[1].item() == amax
 
 
-@pytest.mark.parametrize("M,inter,Kd", [(1, 32, 128), (17, 96, 1552), (37, 1000, 512), (64, 12800, 256), (128, 200, 4096)])
+@pytest.mark.parametrize("M,inter,Kd", [(1, 32, 128), (17, 96, 1552), (37, 1000, 512), (64, 12800, 256), (96, 6144, 256), (128, 200, 4096)])
 def test_fused_swiglu_of_few_rows_equals_gemm_then_swiglu(K, M, inter, Kd):
     """Gate and up rows as two parts of one tile: the f32 sums of these integer operands are exact, so the fused
     epilogue has to give the standalone kernel's bits. Ragged last tiles, K of one block to more than the ring,
