@@ -627,7 +627,12 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     const int et = int(threadIdx.x) - 64;  // 0..127 among the epilogue threads
     uint32_t local = 0;
     bool ok = true;
-    const bool slabs = p.vec != 0 && p.splits == 1;  // the output can be moved by TMA
+    // The output moves by TMA where it can, except the fused SwiGLU of full-width tiles when every CTA has one
+    // tile only: nothing overlaps that epilogue, and its 128 output columns gain less from the slabs than their
+    // hand-overs cost (700 rows, I = 3072, K 4096: 24.8 us stored directly, 26.2 through slabs; 1024 rows, I = 2048
+    // 24.8 and 25.4; 256 rows, I = 6144 24.8 and 25.9). With more tiles the slabs win: 256 rows, I = 12800 34.8 and 33.0,
+    // a chunk of 500 rows through a layer 171.6 and 169.6.
+    const bool slabs = p.vec != 0 && p.splits == 1 && !(p.swiglu_i != 0 && bn == kBN && units <= step);
     SlabState st{tiles_addr + C::kEpiOffset + uint32_t(warp - 2) * (2 * kSlabBytes), ring->res_full[warp - 2], 0u};
     for (int u = first; u < units && ok; u += step, ++local) {
       const int t = u / p.splits, sl = u % p.splits;

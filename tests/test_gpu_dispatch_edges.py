@@ -135,6 +135,20 @@ def test_two_sweep_norm_under_unusual_scales_equals_the_oracle(K, port, rows, co
 
 @pytest.mark.parametrize("M,inter,Kd", [(1, 32, 128), (17, 96, 1552), (37, 1000, 512), (64, 12800, 256), (96, 6144, 256), (128, 200, 4096)])
 def test_fused_swiglu_of_few_rows_equals_gemm_then_swiglu(K, M, inter, Kd):
+    fused_swiglu_case(K, M, inter, Kd)
+
+
+# one tile of 256 columns per CTA pair (stored directly), several, tiles of 128 columns (through slabs), the single
+# form, ragged edges
+@pytest.mark.parametrize("M,inter,Kd,pair", [(700, 3072, 256, True), (1500, 3000, 256, True), (257, 1000, 1552, True), (300, 12800, 256, True),
+                                             (500, 96, 128, True), (129, 1000, 512, False), (300, 3072, 256, False)])
+def test_fused_swiglu_of_many_rows_equals_gemm_then_swiglu(K, monkeypatch, M, inter, Kd, pair):
+    if not pair:
+        monkeypatch.setenv("G4_GEMM_PAIR", "0")
+    fused_swiglu_case(K, M, inter, Kd)
+
+
+def fused_swiglu_case(K, M, inter, Kd):
     """Gate and up rows as two parts of one tile: the f32 sums of these integer operands are exact, so the fused
     epilogue has to give the standalone kernel's bits. Ragged last tiles, K of one block to more than the ring,
     a K that is not whole blocks."""
