@@ -4,12 +4,12 @@ from __future__ import annotations
 import os
 import shutil
 import subprocess
+import sys
 import sysconfig
 
 PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG_DIR, "csrc")
 LIB_PATH = os.path.join(PKG_DIR, "libgranite4_b200.so")
-DISPATCH_PATH = os.path.join(PKG_DIR, "_dispatch.so")  # Python extension: csrc/py_dispatch.cc
 
 SOURCES = ["runtime.cu", "embed.cu", "add_rmsnorm.cu", "rope_kv.cu", "rope_bf16.cu", "swiglu.cu", "decode_glue.cu", "attn_decode.cu", "attn_prefill.cu", "attn_prefill_tc.cu", "gemm_fp8.cu", "kv_pool.cc", "kv_pool_controller.cc", "host_glue.cu"]
 HEADERS = ["g4_host.h", "g4_math.cuh", "g4_tma.cuh", "g4_cluster.cuh", "g4_tcgen05.cuh"]
@@ -28,10 +28,19 @@ def _nvcc() -> str:
     raise RuntimeError("nvcc not found: the CUDA extension cannot be built")
 
 
+def dispatch_path() -> str:
+    """The Python extension (csrc/py_dispatch.cc). It is compiled against one torch and one Python, whose
+    versions its name carries: under another one there is no such file, and an extension built for a different
+    C++ ABI is never loaded."""
+    import torch
+    return os.path.join(PKG_DIR, f"_dispatch-{sys.implementation.cache_tag}-torch{torch.__version__}.so")
+
+
 def is_stale() -> bool:
-    if not os.path.isfile(LIB_PATH) or not os.path.isfile(DISPATCH_PATH):
+    dispatch = dispatch_path()
+    if not os.path.isfile(LIB_PATH) or not os.path.isfile(dispatch):
         return True
-    built = min(os.path.getmtime(LIB_PATH), os.path.getmtime(DISPATCH_PATH))
+    built = min(os.path.getmtime(LIB_PATH), os.path.getmtime(dispatch))
     deps = [os.path.join(CSRC, f) for f in SOURCES + HEADERS + ["py_dispatch.cc"]]
     deps += [os.path.join(PKG_DIR, "..", "include", f) for f in ("granite4_b200.h", "granite4_b200.hpp")]
     return any(os.path.getmtime(d) > built for d in deps)
@@ -46,7 +55,7 @@ def _dispatch_cmd() -> list:
             "-I" + inc, "-I" + os.path.join(inc, "torch", "csrc", "api", "include"),
             "-I" + sysconfig.get_paths()["include"],
             "-I" + os.path.join(os.path.dirname(os.path.dirname(_nvcc())), "include"),
-            os.path.join(CSRC, "py_dispatch.cc"), "-o", DISPATCH_PATH,
+            os.path.join(CSRC, "py_dispatch.cc"), "-o", dispatch_path(),
             "-L" + os.path.join(os.path.dirname(torch.__file__), "lib"), "-ltorch_python", "-ltorch", "-lc10", "-lc10_cuda"]
 
 

@@ -12,10 +12,13 @@ Each call launches on torch's current stream of the tensor's device.
 from __future__ import annotations
 
 import ctypes as C
+import importlib.util
+import os
+import threading
 
 import torch
 
-from . import capi
+from . import _build, capi
 
 
 def _p(t, *dtypes):
@@ -31,17 +34,30 @@ def _p(t, *dtypes):
     return t.data_ptr()
 
 
+_binding = threading.Lock()
+
+
+def _dispatch_module():
+    """The native argument conversion (csrc/py_dispatch.cc), bound to the library capi.py loads."""
+    path = _build.dispatch_path()
+    if not os.path.isfile(path):
+        raise ImportError(f"{path} is missing: the extension has not been built for this torch and Python (_build.build())")
+    spec = importlib.util.spec_from_file_location(__package__ + "._dispatch", path)
+    mod = importlib.util.module_from_spec(spec)
+    lib = capi.lib()
+    mod.bind({fn: C.cast(getattr(lib, fn), C.c_void_p).value for fn in capi.SIGNATURES})
+    return mod
+
+
 class _Unbound:
-    """Stands for the native argument conversion (csrc/py_dispatch.cc) until the first call: binds it
-    to the addresses of the library capi.py loads, then takes its own place."""
+    """Stands for the native argument conversion until the first call, then puts it in its own place."""
 
     def __getattr__(self, name):
         global _n
-        from . import _dispatch
-        lib = capi.lib()
-        _dispatch.bind({fn: C.cast(getattr(lib, fn), C.c_void_p).value for fn in capi.SIGNATURES})
-        _n = _dispatch
-        return getattr(_dispatch, name)
+        with _binding:
+            if _n is self:
+                _n = _dispatch_module()
+        return getattr(_n, name)
 
 
 _n = _Unbound()

@@ -188,6 +188,18 @@ def test_attention_scratch_is_sized_for_the_device_of_the_queries(g4, monkeypatc
         kernels.attn_split_int8(q, u, u, q, q, 1.0, 32, 8, 128, 16, q)
 
 
+def test_an_extension_built_for_another_torch_is_not_loaded(g4, monkeypatch):
+    """The native dispatch is compiled against one torch's C++ ABI: under another version the build counts as stale
+    and the extension that is there is not picked up."""
+    import torch
+    from granite4_b200 import _build, kernels
+    assert not _build.is_stale() and kernels._dispatch_module().__file__ == _build.dispatch_path()
+    monkeypatch.setattr(torch, "__version__", "0.0.1")
+    assert _build.is_stale()
+    with pytest.raises(ImportError, match="torch0.0.1.so is missing"):
+        kernels._dispatch_module()
+
+
 def test_row_table_follows_the_pool_rule(g4):
     from granite4_b200 import paging
     # engine/src/kv_pool.cc:285-298: out[p] = page_id * B + p % B
