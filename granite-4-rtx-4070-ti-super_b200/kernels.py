@@ -209,7 +209,8 @@ def prefill_rope_split_append(qkv, cos_tbl, sin_tbl, base_pos, rows, Hq, Hk, d, 
 
 
 def multi_rows_to_device(desc: capi.MultiRows, device):
-    """Upload a MultiRows descriptor; returns a uint8 CUDA tensor to pass as d_rows."""
+    """Upload a MultiRows descriptor; returns a uint8 CUDA tensor to pass as d_rows. It holds the addresses of the
+    page tables and token arrays only: the caller keeps those tensors alive as long as the descriptor is used."""
     raw = bytes(desc)
     return torch.frombuffer(bytearray(raw), dtype=torch.uint8).to(device)
 
