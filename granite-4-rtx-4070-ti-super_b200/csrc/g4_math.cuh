@@ -83,12 +83,6 @@ __device__ __forceinline__ F32x2 fma2(F32x2 a, F32x2 b, F32x2 c) {
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
   return r;
 }
-__device__ __forceinline__ F32x2 add2(F32x2 a, F32x2 b) {
-  F32x2 r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-
 // ---- running max |x| over packed bf16 pairs -----------------------------------
 // Clearing the two sign bits leaves magnitudes whose bit patterns order like
 // unsigned 16-bit integers, so the running maximum is one AND and one packed

@@ -44,7 +44,7 @@ def test_fp8_codes_of_every_bf16_value_under_every_amax_mantissa(K, port, expone
         assert (got == want).all(), (m, (got != want).sum())
 
 
-def _exact_gemm_case(K, M, N, Kd, kind, pad=0):
+def _exact_gemm_case(K, M, N, Kd, kind, pad=0, in_place=False):
     """Codes from {0, +-1, +-2} make every sum exact in f32, so every form of the GEMM must return the
     integer result exactly (bf16: rounded once), whatever order it adds in."""
     g = torch.Generator(device=DEV).manual_seed(M * 7919 + N * 31 + Kd)
@@ -66,6 +66,9 @@ def _exact_gemm_case(K, M, N, Kd, kind, pad=0):
         rbuf = torch.randint(-8, 8, (M, ldc), generator=g, device=DEV).to(torch.bfloat16)
         res = rbuf[:, :N]
         want = want * 0.5 + res.double()
+        if in_place:
+            rbuf[:, N:] = 7.0
+            buf, out = rbuf, res
     ws = K.gemm_fp8_workspace(M, N, Kd, DEV)
     assert K.gemm_fp8(a, w, out, residual=res, resid_scale=0.5, workspace=ws) == 0
     want = want.float() if kind == "f32" else want.float().to(torch.bfloat16)
@@ -73,13 +76,32 @@ def _exact_gemm_case(K, M, N, Kd, kind, pad=0):
     assert (buf[:, N:] == 7.0).all()  # nothing past column N
 
 
-# row counts at the edges of the forms and of their 128- / 256-row tiles; widths that plan 64, 128, 192 and
-# 256 columns, with ragged last slabs; K of one block, of more blocks than the ring, not a multiple of 128
+# row counts at the edges of the forms and of their 128- / 256-row tiles; widths that plan 64, 128 and 192 columns on
+# CTA pairs, with ragged last slabs; K of one block, of more blocks than the ring, not a multiple of 128
 @pytest.mark.parametrize("M", [1, 8, 9, 16, 17, 33, 128, 129, 255, 256, 257, 500])
 @pytest.mark.parametrize("N,Kd", [(72, 128), (1000, 1552), (4096, 512), (6144, 256)])
 def test_gemm_forms_are_exact_at_their_edges(K, M, N, Kd):
     for kind in ("bf16", "f32", "residual"):
         _exact_gemm_case(K, M, N, Kd, kind, pad=8 if kind == "residual" else 0)
+
+
+def planned_width(M, N, pairs=74):
+    """Columns of a pair tile (csrc/gemm_fp8.cu plan_pair_columns): rounds of tiles over the pairs x measured time."""
+    cost = {w: -(-(-(-M // 256) * -(-N // w)) // pairs) * us for w, us in ((256, 0.33), (192, 0.265), (128, 0.19), (64, 0.16))}
+    best = 256
+    for w in cost:
+        best = w if cost[w] < cost[best] * 0.999 else best
+    return best
+
+
+# every width of a pair tile: one round of tiles and several, ragged rows, the last slab of the last tile ragged
+@pytest.mark.parametrize("M,N,width", [(500, 8192, 256), (2100, 6144, 256), (512, 9208, 256), (500, 6136, 192),
+                                       (300, 4088, 128), (257, 1000, 64)])
+def test_gemm_on_cta_pairs_at_every_tile_width(K, M, N, width):
+    assert planned_width(M, N) == width
+    for kind in ("bf16", "f32", "residual"):
+        _exact_gemm_case(K, M, N, 272, kind, pad=8)
+    _exact_gemm_case(K, M, N, 272, "residual", pad=8, in_place=True)
 
 
 @pytest.mark.parametrize("rows", [1, 2, 3, 5, 8, 9, 15, 16, 17])
