@@ -31,7 +31,7 @@
 //               CTA's own shared memory, no multicast; one 2 KB copy per 16-token page where the
 //               rows are consecutive, else 128 bytes per row) and their scales with 4-byte
 //               cp.async, into a three-stage ring;
-//   warp 1      allocates the tensor memory; one thread issues every MMA and commits them to the
+//   warp 1      allocates the tensor memory; one lane issues every MMA and commits them to the
 //               barriers of whoever waits for the result: per tile, first S of the NEXT tile for both
 //               row tiles (into the S buffer that tile j - 1 used), then P V of this tile for each
 //               row tile as soon as its P is written. The tensor cores thus work on tile j + 1's
@@ -231,7 +231,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_prefill_tc_kernel(const TcPa
   const int hkv = blockIdx.y;
   // a cluster is p.splits consecutive CTAs along x, so this is the rank in it
   const int splits = p.splits, rank = static_cast<int>(blockIdx.x) % splits;
-  // the longest prefixes first
+  // the longest prefixes of a kv head first
   const int blk = (static_cast<int>(gridDim.x) - 1 - static_cast<int>(blockIdx.x)) / splits;
   const int row0 = blk * kCtaPos;                           // first chunk row of this CTA
   const int nrows = min(kCtaPos, p.rows - row0);            // its live rows
@@ -241,7 +241,9 @@ __global__ void __launch_bounds__(kThreads, 1) attn_prefill_tc_kernel(const TcPa
   const int share = static_cast<int>(1ll * n_all * (rank + 1) / splits) - tile0;     // tile0 .. tile0 + share - 1 (may be none)
   // A share that does not begin with tile 0 looks at that tile's logits first, without its P V: the first
   // tile sets the maximum that a row's probabilities are taken against, so they round to f16 as in the unsplit
-  // walk, and the split changes the order of f32 additions only.
+  // walk, and the split changes the order of f32 additions only - unless a later tile exceeds the running maximum
+  // by more than 2^12: that moves the maximum of its own share alone, where the unsplit walk moves it for all that
+  // follows, and the probabilities of the others then round against a smaller maximum (to the same 11 bits).
   const int probe = tile0 > 0 && share > 0 ? 1 : 0;
   const int n_kv = share + probe;  // tiles walked
   auto tile_at = [&](int j) { return j < probe ? 0 : tile0 + j - probe; };
@@ -692,13 +694,15 @@ static int resident_ctas(int splits) {
   return n;
 }
 
-// CTAs per block of query positions. The cost of a plan in cache tiles (~1.3 us): the blocks go over the SMs in
-// rounds, the longest prefixes first, and a round takes its longest block's share plus what a CTA costs beside
-// its tiles (Q rows, first pages, the last P V: kFixed; the look at tile 0 and the exchange: kExchange). Fewer
-// CTAs win a tie. From four rounds on the rounds are full enough and nothing is split. Large clusters lose by
-// themselves: few of them fit between the chip's SM clusters. G4_PREFILL_SPLITS forces a count (tests,
-// measurements). Measured, 128 rows after 4000: 1 CTA per block 93 us, 4 40, 6 33 (the plan), 8 54;
-// 256 rows after 16000: 1 327, 3 127, 4 100 (the plan), 6 141; 1999 rows after 30000: 1 1253 (the plan), 3 1314.
+// CTAs per block of query positions. The cost of a plan in cache tiles (~1.3 us), as if the blocks went over the
+// SMs in rounds, the longest prefixes of all kv heads first: a round takes its longest block's share plus what a CTA
+// costs beside its tiles (Q rows, first pages, the last P V: kFixed; the look at tile 0 and the exchange:
+// kExchange). Fewer CTAs win a tie. (The grid deals out one kv head after the other, so that a short block of one
+// head starts before a long one of the next; the model leaves that out.) From four rounds on the rounds are full
+// enough and nothing is split. Large clusters lose by themselves: few of them fit between the chip's SM clusters.
+// G4_PREFILL_SPLITS forces a count (tests, measurements). Measured, 128 rows after 4000: 1 CTA per block 93 us,
+// 4 40, 6 33 (the plan), 8 54; 256 rows after 16000: 1 327, 3 127, 4 100 (the plan), 6 141; 1999 rows after 30000:
+// 1 1253 (the plan), 3 1314.
 static int plan_splits(int rows, int base_pos, int Hk) {
   constexpr double kFixed = 3.0, kExchange = 3.0;
   if (const char* v = std::getenv("G4_PREFILL_SPLITS"); v != nullptr && std::atoi(v) > 0) {

@@ -19,8 +19,8 @@
 //            swizzle) of the W and A blocks, k-blocks in turn, into a
 //            shared-memory ring;
 //   warp 1   allocates tensor memory; one lane issues tcgen05.mma
-//            (kind::f8f6f4, M 128, N 256, K 32 per instruction) straight from
-//            the ring into one of two 256-column accumulators, and commits each
+//            (kind::f8f6f4, M 128, N 256, K 32 per instruction; the pair form M 256, N as
+//            planned) straight from the ring into one of two 256-column accumulators, and commits each
 //            stage back to the loaders and each finished tile to the epilogue;
 //   warps 2-5 read the finished accumulator out of tensor memory (each warp its
 //            own 32 lanes = 32 output rows), scale, convert and store through
@@ -61,12 +61,11 @@ constexpr int kMaxSplits = 16;
 // epilogue warp, and move by TMA: see store_slabs.
 constexpr uint32_t kSlabBytes = 32 * 128, kEpiBytes = 4 * 2 * kSlabBytes;
 
-// Forms of the kernel; all compute 256 output columns per tile: a stage costs the loader thread
-// about 0.3 us of issue (barrier wait, expect_tx, two TMA instructions) whatever its size, so only
-// 256-row W blocks (32 KB per stage) carry enough bytes per stage to keep up with HBM; 32- and
-// 64-column tiles were measured at a quarter and a half of that rate.
-// kPair = true: the two CTAs of a cluster own a 256 x 256 tile; each loads its 128 rows of A and
-//   its 128 rows of W, and one thread of the leader CTA issues MMAs that run on both SMs
+// Forms of the tiled kernel. The single forms compute 256 output columns per tile, the pair form 64 to 256, as many
+// as make the rounds of tiles over the CTA pairs cheapest (plan_pair_columns): a k-block of a narrow tile costs its
+// four loading threads 0.16 us whatever its size, half of what the MMAs of a 256-column one take.
+// kPair = true: the two CTAs of a cluster own a tile of 256 rows; each loads its 128 rows of A and
+//   its half of the tile's rows of W, and one thread of the leader CTA issues MMAs that run on both SMs
 //   (cta_group::2), so each SM reads half as many W bytes from shared memory per flop.
 // kPair = false: one CTA owns a 128 x 256 tile and both operand blocks. kARows = 16 loads only 16
 //   rows of A per block (decode and verify steps): the MMA still reads 128 rows of shared
@@ -1636,10 +1635,9 @@ extern "C" int granite4_kernel_gemm_fp8(int out_kind, const uint8_t* d_a, long l
     if (rc <= 0) return rc;
   }
   if (M <= kBM) {
-    // A stream of the weights. Measured per layer of four projections (one CUDA graph): the split of
-    // K through the workspace wins at one and two rows (63 us against 70), the full-K stream form
-    // from three rows on (70 us flat up to 16 rows against 74 - 126; 100 - 109 us for 32 - 128 rows
-    // against 121 - 128).
+    // A stream of the weights. Measured per layer of four projections (one CUDA graph), with the 16-row form off: the
+    // split of K through the workspace 58 us at one and two rows, 68 - 126 at 3 - 16; the full-K stream form 57 up
+    // to 16 rows, 64 at 32, 69 at 64, 92 at 128 (the tiled form there: 96, 97, 99).
     const SplitPlan pl = plan_split(M, N, K, sm_count());
     const bool can_split = pl.splits > 1 && d_ws != nullptr && ws_bytes >= static_cast<long long>(pl.bytes);
     if (stream_enabled() && !(M <= 2 && can_split)) return launch_stream(fn, d_a, lda, d_w, p);
