@@ -501,8 +501,11 @@ int attn_prefill_flash(const char* fn, const uint16_t* d_q, float scale, int Hq,
   p.q = d_q, p.ck = d_ck, p.cv = d_cv, p.ks = d_ks, p.vs = d_vs, p.pt = d_pt, p.out = d_out;
   p.rows = rows, p.base_pos = base_pos, p.Hq = Hq, p.Hk = Hk, p.stride = stride;
   p.scale_log2 = scale * 1.4426950408889634f;
-  const char* v = std::getenv("G4_PREFILL_ROWS32");  // 0: 16 query positions per CTA
-  if (!(v != nullptr && v[0] == '0')) {
+  // Below 64 rows a few CTAs walk the whole prefix, and one head per CTA spreads them over more SMs. A longer chunk
+  // has CTAs enough: there the conversion of K and V is shared by four heads (2048 rows 209 us, 384 with one head per
+  // CTA; 8192 rows 2.36 ms and 5.3). G4_PREFILL_ROWS32=0: 16 positions and four heads always.
+  const char* v = std::getenv("G4_PREFILL_ROWS32");
+  if (rows < 64 && !(v != nullptr && v[0] == '0')) {
     const dim3 grid(static_cast<unsigned>((rows + kQRows2 - 1) / kQRows2), static_cast<unsigned>(Hq));
     G4_LAUNCH_PDL(fn, attn_prefill2_kernel, grid, dim3(kWarps2 * 32), sizeof(PrefillSmem2), current_stream(), p);
     return 0;

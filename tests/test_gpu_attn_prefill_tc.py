@@ -186,6 +186,20 @@ def test_output_that_is_not_16_byte_aligned(K):
     assert close(f32_of(got), f32_of(want), 0.01) and int(buf[:2].abs().sum()) == 0 and int(buf[-6:].abs().sum()) == 0
 
 
+# what an output off the 16-byte boundary takes: one head per CTA below 64 rows, four from there on
+@pytest.mark.parametrize("rows,base", [(63, 300), (64, 300), (65, 0), (200, 1000)])
+def test_chunks_around_the_change_of_the_mma_sync_form(K, monkeypatch, rows, base):
+    stride = 2048
+    pl = pool(rows, stride)
+    rng = np.random.default_rng(rows + base)
+    q = bf16_bits(2.0 * rng.standard_normal((rows, Hq * D)))
+    monkeypatch.setenv("G4_PREFILL_TC", "0")
+    got = run(K, q, pl, base, stride, None)
+    sel = np.unique([0, 1, 15, 16, 31, 32, 47, 48, rows - 1])
+    exact = f64_rows(q[sel], pl, [np.arange(stride, dtype=np.int32)] * len(sel), (base + sel).astype(np.int32))
+    assert close(f32_of(got[sel]).reshape(len(sel), Hq, D), exact, 0.01)
+
+
 @pytest.mark.parametrize("rows,base", [(32, 0), (33, 1000), (48, 63), (63, 1985)])
 def test_chunks_below_the_tensor_core_form(K, rows, base):
     """32 - 63 rows (one query head, two row tiles and two halves of the dims per CTA): ragged row tiles, rows whose
