@@ -684,7 +684,10 @@ int attn_launch(const char* fn, const uint16_t* d_q, const int8_t* d_cache_k, co
   SplitPlan s = plan_splits(rows, rows_per_group, Hk, max_len);
   if (r.d_row_grp != nullptr) s = plan_splits_for_groups(r.ngroups, rows_per_group, Hk, max_len);
   const long long need = scratch_bytes_of(s, Hk);
-  if (s.splits > 1 && single_split_without_scratch && (d_scratch == nullptr || scratch_bytes < need)) {
+  // the merge of the splits stores eight bytes at a time; one split stores single values
+  const bool whole = reinterpret_cast<uintptr_t>(d_out) % 8 != 0 ||
+                     (single_split_without_scratch && (d_scratch == nullptr || scratch_bytes < need));
+  if (s.splits > 1 && whole) {
     s.splits = 1;
     s.split_len = (max_len + kSplitAlign - 1) / kSplitAlign * kSplitAlign;
   }
@@ -804,9 +807,10 @@ int granite4_prefill_attention_int8(const uint16_t* d_q_rot, float scale, int Hq
   if (base_pos < 0 || rows <= 0 || base_pos > INT_MAX - rows) return g4::fail(fn, "invalid arguments");
   // A chunk of 32 rows or more takes the flash form (one K / V tile serves 16 positions x 4 heads);
   // shorter ones the decode kernel as groups of four rows, which can also split a long context
-  // over CTAs. G4_PREFILL_FLASH=0 keeps every chunk on the decode kernel.
+  // over CTAs, and any with an output between two words. G4_PREFILL_FLASH=0 keeps every chunk on the decode kernel.
   const char* flash_env = std::getenv("G4_PREFILL_FLASH");
-  if (rows >= 32 && !(flash_env != nullptr && flash_env[0] == '0')) {
+  const bool words = reinterpret_cast<uintptr_t>(d_out) % 4 == 0;  // the flash forms store four bytes at a time or more
+  if (rows >= 32 && words && !(flash_env != nullptr && flash_env[0] == '0')) {
     if (d_q_rot == nullptr || d_cache_k8 == nullptr || d_cache_v8 == nullptr || d_k_scale == nullptr ||
         d_v_scale == nullptr || d_out == nullptr || stride <= 0 || base_pos + rows > stride || !std::isfinite(scale))
       return g4::fail(fn, "invalid arguments");

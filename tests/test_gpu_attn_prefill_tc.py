@@ -173,17 +173,32 @@ def test_cache_range_split_over_a_cluster(K, monkeypatch, rows, base, splits, si
     assert close(f32_of(got[sel]).reshape(len(sel), Hq, D), exact, tol)
 
 
-def test_output_that_is_not_16_byte_aligned(K):
-    """An output on a 4-byte boundary is taken by the kernels that store four bytes at a time."""
-    rows, stride = 64, 128
+@pytest.mark.parametrize("rows,at", [(64, 2), (64, 1), (33, 1), (20, 1)])
+def test_output_that_is_not_16_byte_aligned(K, rows, at):
+    """An output on a 4-byte boundary is taken by the kernels that store four bytes at a time, one on a 2-byte
+    boundary by the decode kernel, which stores single values."""
+    stride = 128
     pl = pool(3, stride)
     q = bf16_bits(np.random.default_rng(4).standard_normal((rows, Hq * D)))
     want = run(K, q, pl, 0, stride, None)
     buf = torch.zeros(rows * Hq * D + 8, dtype=torch.int16, device=DEV)
-    out = buf[2:2 + rows * Hq * D].view(rows, Hq * D)
+    out = buf[at:at + rows * Hq * D].view(rows, Hq * D)
     assert K.prefill_attention_int8(dev(q), SCALE, Hq, Hk, D, 0, stride, out, *[dev(x) for x in pl], pt=None) == 0
     got = out.cpu().numpy().view(np.uint16)
-    assert close(f32_of(got), f32_of(want), 0.01) and int(buf[:2].abs().sum()) == 0 and int(buf[-6:].abs().sum()) == 0
+    assert close(f32_of(got), f32_of(want), 0.01) and int(buf[:at].abs().sum()) == 0 and int(buf[at + rows * Hq * D:].abs().sum()) == 0
+
+
+def test_decode_output_that_is_not_8_byte_aligned(K):
+    """A context long enough to be split: the merge of the splits stores eight bytes at a time, so this one is not."""
+    ctx, stride = 1500, 1536
+    pl = [dev(x) for x in pool(9, stride)]
+    q = dev(bf16_bits(np.random.default_rng(9).standard_normal((1, Hq * D))))
+    pos = torch.tensor([ctx], dtype=torch.int32, device=DEV)
+    want, buf = torch.empty(1, Hq * D, dtype=torch.int16, device=DEV), torch.zeros(Hq * D + 8, dtype=torch.int16, device=DEV)
+    for out in (want, buf[1:1 + Hq * D].view(1, Hq * D)):
+        assert K.attn_decode_int8_paged(q, *pl, pos, Hq, Hk, D, stride, stride, SCALE, out) == 0
+    assert close(f32_of(buf[1:1 + Hq * D].cpu().numpy().view(np.uint16)), f32_of(want[0].cpu().numpy().view(np.uint16)), 0.01)
+    assert int(buf[:1].abs().sum()) == 0 and int(buf[1 + Hq * D:].abs().sum()) == 0
 
 
 # what an output off the 16-byte boundary takes: one head per CTA below 64 rows, four from there on
