@@ -398,7 +398,7 @@ __device__ __forceinline__ void residual_ahead(const CUtensorMap* map_res, const
 
 // Columns n0 .. n_end - 1 of rows row0 .. row0 + 31 (row0 < M; n0 < n_end <= N) from the accumulator at
 // taddr. Returns the running max |.| of the fused SwiGLU's outputs (packed bf16 pairs; of stored elements
-// only: rows and columns past the output are zero in the accumulator). ok: false once a wait ran out.
+// only). ok: false once a wait ran out.
 __device__ __forceinline__ uint32_t store_slabs(const GemmParams& p, const CUtensorMap* map_out, const CUtensorMap* map_res,
                                                 SlabState& st, Ring* ring, uint32_t taddr, int lane, int row0, int n0,
                                                 int n_end, int half, float a_scale, bool& ok) {
@@ -448,7 +448,7 @@ __device__ __forceinline__ uint32_t store_slabs(const GemmParams& p, const CUten
         for (int j = 0; j < 32; j += 8) {
           const uint4 w = make_uint4(pack_bf16x2(a[j], a[j + 1]), pack_bf16x2(a[j + 2], a[j + 3]), pack_bf16x2(a[j + 4], a[j + 5]),
                                      pack_bf16x2(a[j + 6], a[j + 7]));
-          amax = amax_acc(amax, w);
+          if (row0 + lane < p.M) amax = amax_acc(amax, w);  // rows past M: zero times a scale that may be infinite
           slab_put(slab_at(slab, lane, h * 4 + j / 8), w);
         }
         continue;

@@ -170,6 +170,19 @@ def test_fused_swiglu_of_many_rows_equals_gemm_then_swiglu(K, monkeypatch, M, in
     fused_swiglu_case(K, M, inter, Kd)
 
 
+@pytest.mark.parametrize("M,inter", [(17, 96), (100, 12800), (257, 1000), (300, 12800), (700, 3072)])
+def test_fused_swiglu_amax_is_of_the_rows_that_exist(K, M, inter):
+    """An infinite activation scale: the stored values and their maximum are infinite, whatever rows past M would be."""
+    a, w = (torch.full((r, 128), 0x38, dtype=torch.uint8, device=DEV) for r in (M, 2 * inter))  # all 1.0
+    out, slot = torch.empty(M, inter, dtype=torch.bfloat16, device=DEV), torch.full((2,), 9.0, device=DEV)
+    inf = torch.tensor([float("inf"), 0.0], device=DEV)
+    assert K.gemm_fp8(a, w, out, a_scale=inf, swiglu_scale_amax=slot) == 0
+    both = torch.full((M, inter), float("inf"), device=DEV)
+    want, c8, sa = torch.empty_like(out), torch.empty(M, inter, dtype=torch.uint8, device=DEV), torch.zeros(2, device=DEV)
+    assert K.swiglu_fp8(both, both, want, c8, sa) == 0
+    assert torch.equal(out.view(torch.int16), want.view(torch.int16)) and slot[1].item() == sa[1].item() == float("inf")
+
+
 def fused_swiglu_case(K, M, inter, Kd):
     """Gate and up rows as two parts of one tile: the f32 sums of these integer operands are exact, so the fused
     epilogue has to give the standalone kernel's bits. Ragged last tiles, K of one block to more than the ring,
